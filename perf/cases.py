@@ -3,8 +3,8 @@ library do, through the calls it makes (volvoxai_b200.w8a8), over the range of s
 
 ``listed()`` names twelve cases, ``draw(rng)`` gives more of the same ranges, ``prepare(case, seed)`` makes
 the inputs and the weights a program holds before the call, ``run(state)`` is one pass, ``work(case)`` the
-bytes and operations no implementation can do without and ``tolerance(case)`` how far another correct
-implementation's outputs may lie.
+bytes and operations no implementation can do without, ``tolerance(case)`` how far another correct
+implementation's outputs may lie and ``exact(case, seed)`` the floating outputs of ``run`` in 64 bits.
 
 Kinds of a case:
   f32      one linear, fp32 in and fp32 out (dynamic per-token quantization, dequantization, bias)
@@ -128,11 +128,15 @@ def _scales(g, n, top=127):
     return (_SIGMA * _PEAK / top) * (0.9 + 0.2 * torch.rand(n, generator=g, device="cuda"))
 
 
-def _weight(ctx, g, n, k, bias=False, bias_i32=False):
+def _drawn(g, n, k, bias=False, bias_i32=False):
     w, ws = _codes(g, n, k), _scales(g, n)
     bf = torch.randn(n, generator=g, device="cuda") * 0.01 if bias else None
     bi = torch.randint(-2000, 2001, (n,), generator=g, device="cuda", dtype=torch.int32) if bias_i32 else None
-    host = [None if t is None else t.cpu().numpy() for t in (w, ws, bf, bi)]
+    return w, ws, bf, bi
+
+
+def _weight(ctx, g, n, k, bias=False, bias_i32=False):
+    host = [None if t is None else t.cpu().numpy() for t in _drawn(g, n, k, bias, bias_i32)]
     return w8a8.Weight.from_i8(ctx, *host)
 
 
@@ -147,14 +151,29 @@ def _pack_words(codes, bits):
     return torch.where(words >= 2 ** 31, words - 2 ** 32, words).to(torch.int32)
 
 
-def _grouped_weight(ctx, g, case):
+def _grouped_drawn(g, case):
     n, k, bits, group = case["n"], case["k"], case["bits"], case["group"]
     top = 127 if bits == 8 else 7
-    words = torch.cat([_pack_words(_codes(g, min(2048, n - lo), k, top), bits) for lo in range(0, n, 2048)])
+    codes = torch.cat([_codes(g, min(2048, n - lo), k, top) for lo in range(0, n, 2048)])
     scales = _scales(g, n * ((k + group - 1) // group), top).view(n, -1)
-    bias = (torch.randn(n, generator=g, device="cuda") * 0.01).cpu().numpy() if case["bias"] else None
+    return codes, scales, torch.randn(n, generator=g, device="cuda") * 0.01 if case["bias"] else None
+
+
+def _grouped_weight(ctx, g, case):
+    n, bits = case["n"], case["bits"]
+    codes, scales, bias = _grouped_drawn(g, case)
+    words = torch.cat([_pack_words(codes[lo:lo + 2048], bits) for lo in range(0, n, 2048)])
     make = w8a8.Weight.from_w8_words if bits == 8 else w8a8.Weight.from_w4_words
-    return make(ctx, words.cpu().numpy(), scales.cpu().numpy(), k, group, bias)
+    return make(ctx, words.cpu().numpy(), scales.cpu().numpy(), case["k"], case["group"],
+                None if bias is None else bias.cpu().numpy())
+
+
+def _layer_inputs(g, case):
+    rows, hidden = case["rows"], case["hidden"]
+    x = torch.randn((rows, hidden), generator=g, device="cuda")
+    attn = torch.randn((rows, case["attn"]), generator=g, device="cuda") * 0.5
+    norms = [1.0 + 0.1 * torch.randn(hidden, generator=g, device="cuda") for _ in range(2)]
+    return x, attn, *norms
 
 
 def _out_scale(k):
@@ -171,10 +190,7 @@ def prepare(case, seed):
     s = {"kind": kind, "ctx": ctx}
     if kind == "layer":
         hidden, attn, kv, inter = case["hidden"], case["attn"], case["kv"], case["inter"]
-        s["x"] = torch.randn((rows, hidden), generator=g, device="cuda")
-        s["attn"] = torch.randn((rows, attn), generator=g, device="cuda") * 0.5
-        s["norm1"] = 1.0 + 0.1 * torch.randn(hidden, generator=g, device="cuda")
-        s["norm2"] = 1.0 + 0.1 * torch.randn(hidden, generator=g, device="cuda")
+        s["x"], s["attn"], s["norm1"], s["norm2"] = _layer_inputs(g, case)
         s["qkv"] = _weight(ctx, g, attn + 2 * kv, hidden)
         s["o"] = _weight(ctx, g, hidden, attn)
         s["gate_up"] = _weight(ctx, g, 2 * inter, hidden)       # channels interleaved (gate_0, up_0, gate_1, ...)
@@ -229,6 +245,57 @@ def run(s):
     mid2 = ctx.requantize_linear(mid, *s["mid"], *s["mid2"])
     out = ctx.qlinear_device(s["down"], mid2, *s["mid2"], *s["out"])
     return {"mid": mid, "q": out, "y": ctx.dequantize_linear(out, *s["out"])}
+
+
+# ---- the floating outputs in 64 bits --------------------------------------------------------------
+
+def _quantized(x):
+    """The row's code and scale are defined in 32 bits (x and scale are fp32, the quotient is rounded to fp32, then
+    to the nearest even whole number); a quotient taken in 64 bits and rounded to 32 is that fp32 quotient."""
+    scale = (x.abs().amax(dim=1, keepdim=True).double() / 127.0).float()
+    scale = torch.where(scale == 0, torch.ones_like(scale), scale)
+    return (x.double() / scale.double()).float().round().clamp(-127, 127).double(), scale.double()
+
+
+def _linear64(x, w, ws, bias=None):
+    q, scale = _quantized(x)
+    y = (q @ w.double().T) * scale * ws.double()
+    return y if bias is None else y + bias.double()
+
+
+def _norm64(x, weight):
+    x = x.double()
+    return (x / (x.square().mean(dim=1, keepdim=True) + _EPS).sqrt() * weight.double()).float()
+
+
+def exact(case, seed):
+    """What ``run`` returns in 64 bits, from the codes that the storage holds.  A linear's input is fp32, so a layer's
+    outputs are rounded where the next linear takes them up.  None where outputs are codes: those are exact."""
+    g, kind, rows = _gen(seed), case["kind"], case["rows"]
+    if kind == "f32":
+        w, ws, bias, _ = _drawn(g, case["n"], case["k"], bias=case["bias"])
+        return _linear64(_activations(g, rows, case["k"]), w, ws, bias)
+    if kind == "grouped":
+        codes, scales, bias = _grouped_drawn(g, case)
+        q, scale = _quantized(_activations(g, rows, case["k"]))
+        k, group = case["k"], case["group"]
+        y = torch.zeros((rows, case["n"]), dtype=torch.float64, device="cuda")
+        for i, lo in enumerate(range(0, k, group)):
+            hi = min(k, lo + group)
+            y += (q[:, lo:hi] @ codes[:, lo:hi].double().T) * scales[:, i].double()
+        y *= scale
+        return y if bias is None else y + bias.double()
+    if kind == "layer":
+        hidden, attn, kv, inter = case["hidden"], case["attn"], case["kv"], case["inter"]
+        x, a, norm1, norm2 = _layer_inputs(g, case)
+        weights = [_drawn(g, n, k)[:2] for n, k in ((attn + 2 * kv, hidden), (hidden, attn), (2 * inter, hidden), (hidden, inter))]
+        qkv = _linear64(_norm64(x, norm1), *weights[0])
+        h = _linear64(a, *weights[1]) + x.double()
+        gate_up = _linear64(_norm64(h.float(), norm2), *weights[2])
+        act = torch.nn.functional.silu(gate_up[:, 0::2]) * gate_up[:, 1::2]
+        y = _linear64(act.float(), *weights[3]) + h
+        return {"qkv": qkv, "h": h, "act": act, "y": y}
+    return None
 
 
 # ---- what one pass cannot do without ------------------------------------------------------------
