@@ -25,6 +25,7 @@
 // destination each). All mbarrier waits are bounded; a CTA that gives up raises
 // the status word and tells its partner, and both drain, free their TMEM and return.
 #include "tcgen05.cuh"
+#include "store_tile.cuh"
 
 namespace vxb {
 
@@ -273,6 +274,8 @@ __device__ __forceinline__ void gemm_i8_pair_body(const GemmTcgen05Args& args) {
         float* s_bias = sm.bias() + (warp - 2u) * kEpiCols;
         const float zero_f = __int2float_rn(ep.out_zero);
         const float lo_f = __int2float_rn(ep.out_lo), hi_f = __int2float_rn(ep.out_hi);
+        // every 32-column chunk of a row starts on 16 bytes (a chunk of the SiLU * Mul tail is 16 outputs wide)
+        const bool aligned = (((uintptr_t)ep.out | (ep.mode == kEpiI8 ? (uintptr_t)ep.ld : (uintptr_t)ep.ld * 4u)) & 15u) == 0;
         const bool sat_s8 = ep.out_lo == -128 && ep.out_hi == 127, sat_u8 = ep.out_lo == 0 && ep.out_hi == 255;
         uint32_t acc = 0, acc_phase = 0;
         bool ok = true;
@@ -301,7 +304,7 @@ __device__ __forceinline__ void gemm_i8_pair_body(const GemmTcgen05Args& args) {
 
             const uint32_t row = m0 + quarter * 32 + lane;
             const bool row_ok = row < args.rows;
-            const float as = (row_ok && ep.mode != kEpiAcc) ? __ldg(ep.row_scales + row) : 0.0f;
+            const float as = (row_ok && ep.mode != kEpiAcc) ? __ldg(ep.row_scales + row) : 1.0f;   // (rows beyond the batch: any scale)
             const bool fast = ep.fast_div != 0 && div_const_row_ok(as);
             const uint32_t taddr = tmem_base + ((quarter * 32u) << 16) + acc * kAccCols + cbase;
 #pragma unroll 1
@@ -310,7 +313,6 @@ __device__ __forceinline__ void gemm_i8_pair_body(const GemmTcgen05Args& args) {
                 tmem_ld32(taddr + c, r);
                 tmem_ld_wait();
                 const uint32_t col = n0 + c;
-                const bool wide = ep.mode != kEpiI8;                // 32-bit outputs go through the staging below
                 if (gather) {
                     // no early exit: the destination's tensor map clips rows beyond the batch and columns beyond
                     // the shard.  A new group of 64 columns starts once the previous group's stores have left the tile.
@@ -320,9 +322,13 @@ __device__ __forceinline__ void gemm_i8_pair_body(const GemmTcgen05Args& args) {
                     }
                 } else {
                     if (col >= args.n) continue;                   // uniform over the warp
-                    if (!row_ok && !wide) continue;
                 }
                 const bool full = col + 32 <= args.n;
+                // this warp's store tile, its first row and how many of its 32 rows exist (made where they are used:
+                // held throughout the loop they cost registers that the epilogue needs)
+                auto store_tile = [&] { return sm.base + kOffStore + (warp - 2u) * kStoreBytes; };
+                auto first_row = [&] { return m0 + quarter * 32u; };
+                auto live_rows = [&] { const uint32_t r0 = first_row(); return r0 >= args.rows ? 0u : args.rows - r0 < 32u ? args.rows - r0 : 32u; };
                 const float4* w4 = reinterpret_cast<const float4*>(s_ws + c);
                 const float4* b4 = reinterpret_cast<const float4*>(s_bias + c);
                 if (ep.mode == kEpiI8) {
@@ -403,13 +409,22 @@ __device__ __forceinline__ void gemm_i8_pair_body(const GemmTcgen05Args& args) {
                                 tma_store_commit();
                             }
                         }
-                    } else if (full && (((uintptr_t)dst) & 15u) == 0) {
-                        reinterpret_cast<uint4*>(dst)[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-                        reinterpret_cast<uint4*>(dst)[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
+                    } else if (full && aligned) {
+                        if (row_ok) {
+                            reinterpret_cast<uint4*>(dst)[0] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+                            reinterpret_cast<uint4*>(dst)[1] = make_uint4(packed[4], packed[5], packed[6], packed[7]);
+                        }
                     } else {
-#pragma unroll
-                        for (int i = 0; i < 32; i++)
-                            if (col + i < args.n) dst[i] = (int8_t)((packed[i >> 2] >> (8 * (i & 3))) & 0xffu);
+                        // a ragged edge or rows that start on any byte: 64 columns at a time through the warp's tile
+                        const uint32_t g = c & ~63u;
+                        const bool alone = (c & 32u) && aligned;   // the chunk before this one was stored directly
+                        if (!(c & 32u) || alone) __syncwarp();
+                        stage_bytes(store_tile(), lane, alone ? 0u : (c >> 5) & 1u, packed);
+                        if ((c & 32u) || col + 32 >= args.n) {
+                            const uint32_t first = alone ? c : g, left = args.n - (n0 + first);
+                            __syncwarp();
+                            flush_bytes(store_tile(), lane, (int8_t*)ep.out + (size_t)first_row() * ep.ld + n0 + first, ep.ld, live_rows(), left < 64u ? left : 64u);
+                        }
                     }
                 } else {
                     uint32_t o[32];
@@ -445,48 +460,12 @@ __device__ __forceinline__ void gemm_i8_pair_body(const GemmTcgen05Args& args) {
                     }
                     if (ep.mode == kEpiF32 && ep.act == 1u) {
                         // channel pairs (gate, up) -> silu(gate) * up, one output column per pair
-                        if (row_ok) {
-                            float* dst = (float*)ep.out + (size_t)row * ep.ld + (col >> 1);
+                        float y[16];
 #pragma unroll
-                            for (int j = 0; j < 16; j++)
-                                if (col + 2 * j + 1 < args.n)
-                                    dst[j] = epi_silu_mul(__uint_as_float(o[2 * j]), __uint_as_float(o[2 * j + 1]));
-                        }
-                        continue;
-                    }
-                    // Each thread holds 128 contiguous bytes of its own row; stored directly, one store
-                    // instruction touches 32 different rows. Instead the warp passes 16 rows at a time
-                    // through shared memory (16-byte pieces XOR-swizzled by row: no bank conflicts either
-                    // way) and stores whole 128-byte row segments, four rows per instruction.
-                    uint8_t* stage = sm.base + kOffStore + (warp - 2u) * kStoreBytes;
-#pragma unroll
-                    for (uint32_t half16 = 0; half16 < 2; half16++) {
-                        __syncwarp();
-                        if ((lane >> 4) == half16) {
-                            uint8_t* mine = stage + (lane & 15u) * 128u;
-#pragma unroll
-                            for (uint32_t j = 0; j < 8; j++)
-                                *reinterpret_cast<uint4*>(mine + ((j ^ (lane & 7u)) << 4)) =
-                                    make_uint4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
-                        }
-                        __syncwarp();
-                        const uint32_t piece = lane & 7u;
-#pragma unroll
-                        for (uint32_t i = 0; i < 4; i++) {
-                            const uint32_t rl = 4u * i + (lane >> 3);                 // row within the 16
-                            const uint4 v = *reinterpret_cast<const uint4*>(stage + rl * 128u + ((piece ^ (rl & 7u)) << 4));
-                            const uint32_t grow = m0 + quarter * 32u + half16 * 16u + rl, gcol = col + piece * 4u;
-                            if (grow >= args.rows || gcol >= args.n) continue;
-                            uint32_t* dst = (uint32_t*)ep.out + (size_t)grow * ep.ld + gcol;
-                            if (gcol + 4u <= args.n && (((uintptr_t)dst) & 15u) == 0) {
-                                *reinterpret_cast<uint4*>(dst) = v;
-                            } else {
-                                const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-                                for (uint32_t e = 0; e < 4; e++)
-                                    if (gcol + e < args.n) dst[e] = w[e];
-                            }
-                        }
+                        for (int j = 0; j < 16; j++) y[j] = epi_silu_mul(__uint_as_float(o[2 * j]), __uint_as_float(o[2 * j + 1]));
+                        store_half_words(store_tile(), lane, y, (float*)ep.out + (size_t)first_row() * ep.ld + (col >> 1), ep.ld, live_rows(), (args.n - col) >> 1, full && aligned);
+                    } else {
+                        store_words(store_tile(), lane, o, (uint32_t*)ep.out + (size_t)first_row() * ep.ld + col, ep.ld, live_rows(), args.n - col, full && aligned);
                     }
                 }
             }
