@@ -107,7 +107,7 @@ typedef struct VxbPlanQuery {
 /* Per-row quantizer (K1) chosen for calls that start from fp32 activations. */
 typedef enum VxbQuantizerId {
     VXB_QUANTIZER_NONE = 0,   /* prepared int8 activations, or quantization fused into the GEMV */
-    VXB_QUANTIZER_SCALAR,     /* quantize_rows_scalar: any width / alignment, one warp per row */
+    VXB_QUANTIZER_SCALAR,     /* quantize_rows_any: any width / alignment, 32..256 threads per row */
     VXB_QUANTIZER_VEC,        /* quantize_rows_vec<TPR>: row cached in registers, 128-bit loads */
     VXB_QUANTIZER_CLUSTER     /* quantize_rows_cluster<S>: few long rows shared by 2/4/8 CTAs */
 } VxbQuantizerId;

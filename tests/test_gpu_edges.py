@@ -15,6 +15,29 @@ def bits(a):
     return a.view(np.uint32)
 
 
+@pytest.mark.parametrize("k", [1, 31, 33, 257, 1023, 1025, 2047, 4097, 8190, 8195])
+@pytest.mark.parametrize("rows", [1, 3, 700])
+def test_quantizer_any_width_and_alignment(torch, ctx, oracle, k, rows):
+    """Widths around the threads-per-row steps of the any-alignment quantizer, on a base 4 bytes off; an invalid, a
+    zero, a very small and a very large row."""
+    rng = np.random.default_rng(k * 3 + rows)
+    x = rng.standard_normal((rows, k)).astype(np.float32)
+    if rows > 4:
+        x[1] = 0
+        x[2, k // 2] = np.inf
+        x[3] *= np.float32(1e-35)
+        x[4] *= np.float32(1e30)
+    qo, so, vo = oracle.quantize_rows(x)
+    flat = torch.empty(rows * k + 1, device="cuda")
+    flat[1:] = dev(torch, x).flatten()
+    kpad = (k + 127) // 128 * 128
+    q, s, v = ctx.quantize_rows(flat[1:].view(rows, k), ldq=kpad)
+    q, s, v = q.cpu().numpy(), s.cpu().numpy(), v.cpu().numpy()
+    assert np.array_equal(v != 0, vo != 0)
+    assert np.array_equal(q[:, :k], qo) and (q[:, k:] == 0).all()
+    assert np.array_equal(bits(s[vo != 0]), bits(so[vo != 0])) and np.isnan(s[vo == 0]).all()
+
+
 @pytest.mark.parametrize("n", [1, 3, 31, 33, 62, 64, 66, 97, 129, 250, 257, 514])
 @pytest.mark.parametrize("rows,lead,extra", [(129, 0, 0), (161, 1, 2), (300, 2, 5), (140, 16, 32), (131, 4, 8)])
 def test_byte_outputs_on_any_boundary(torch, ctx, n, rows, lead, extra):
@@ -57,3 +80,21 @@ def test_word_outputs_on_any_boundary(torch, ctx, n, lead):
     assert (wide[:, lead:lead + n // 2].double() - y).abs().le(1e-6 * y.abs() + 1e-30).all()
     assert (wide[:, :lead] == 99).all() and (wide[:, lead + n // 2:] == 99).all()
     weight.close()
+
+
+@pytest.mark.parametrize("rows,k", [(1, 64), (5, 1000), (64, 1024), (700, 576), (40, 9000)])
+def test_rmsnorm_products_near_and_far_from_one(torch, ctx, rows, k):
+    """The normalized rows against the same arithmetic in 64 bits: ordinary rows, rows scaled to 1e-25 and 1e25 (the
+    products leave the range of the split form), gammas of 0, 1e-33 and 1e30."""
+    rng = np.random.default_rng(rows + k)
+    x = rng.standard_normal((rows, k)).astype(np.float32)
+    x[rows // 2] *= np.float32(1e-25)
+    x[rows // 3] *= np.float32(1e25 if rows > 3 else 1)
+    g = (1 + 0.1 * rng.standard_normal(k)).astype(np.float32)
+    g[:4] = 0, 1e-33, 1e30, -1
+    y, q, s, v = ctx.rmsnorm_quantize_rows(dev(torch, x), dev(torch, g), 1e-30, ldq=(k + 127) // 128 * 128)
+    x64 = x.astype(np.float64)
+    want = (x64 / np.sqrt((x64 ** 2).mean(axis=1, keepdims=True) + float(np.float32(1e-30))) * g.astype(np.float64)).astype(np.float32)
+    y = y.cpu().numpy()
+    # one rounding to fp32 each; a 64-bit rounding can tip it in a handful of elements, by one place
+    assert (np.abs(y.view(np.int32).astype(np.int64) - want.view(np.int32)) <= 1).all() and (y != want).mean() <= 1e-4

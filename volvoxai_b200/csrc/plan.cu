@@ -123,7 +123,7 @@ void plan_quantizer(const VxbPlanQuery& q, VxbLaunchPlan* p) {
     p->workspace_bytes += (uint64_t)q.rows * kpad + (uint64_t)q.rows * 4;
     p->launches += 1;
     if (q.k % 4 != 0) {
-        p->quantizer = VXB_QUANTIZER_SCALAR; p->quantizer_grid = ceil_div(q.rows, 8); p->quantizer_cluster = 1;
+        p->quantizer = VXB_QUANTIZER_SCALAR; p->quantizer_grid = ceil_div(q.rows, 256 / quantize_any_threads(q.rows, q.k)); p->quantizer_cluster = 1;
         return;
     }
     const uint32_t words = kpad / 4;
@@ -134,7 +134,7 @@ void plan_quantizer(const VxbPlanQuery& q, VxbLaunchPlan* p) {
         p->quantizer_grid = p->quantizer_cluster * q.rows;
         return;
     }
-    const uint32_t tpr = q.k <= 256 ? 8 : q.k <= 1024 ? 32 : q.k <= 2048 ? 64 : q.k <= 4096 ? 128 : 256;
+    const uint32_t tpr = quantize_vec_threads(q.rows, q.k);
     p->quantizer = VXB_QUANTIZER_VEC; p->quantizer_cluster = 1;
     p->quantizer_grid = ceil_div(q.rows, 256 / tpr);
 }
