@@ -82,6 +82,52 @@ def test_word_outputs_on_any_boundary(torch, ctx, n, lead):
     weight.close()
 
 
+@pytest.mark.parametrize("in_u8", [False, True])
+@pytest.mark.parametrize("rows,k,n", [(1, 128, 40), (40, 48, 33), (128, 256, 130), (130, 16, 65), (200, 1283, 50), (300, 576, 1536),
+                                      (700, 2064, 300)])
+def test_static_rows_in_place_and_padded(torch, ctx, oracle, in_u8, rows, k, n):
+    """Codes read where they are (whole 16-byte pieces) or through the padded layout, with and without a zero point,
+    from an unaligned base, and with the output lying over the input."""
+    from volvoxai_b200 import w8a8
+    rng = np.random.default_rng(rows + k + n + in_u8)
+    x = rng.integers(0, 256, size=(rows, k)).astype(np.uint8) if in_u8 else rng.integers(-128, 128, size=(rows, k)).astype(np.int8)
+    w = rng.integers(-127, 128, size=(n, k), dtype=np.int8)
+    ws = rng.uniform(0.001, 0.02, size=n).astype(np.float32)
+    b = rng.integers(-500, 500, size=n).astype(np.int32)
+    weight = w8a8.Weight.from_i8(ctx, w, ws, bias_i32=b)
+    for zero in ((128, 7) if in_u8 else (0, -9)):
+        want = oracle.qlinear_i8u8(x, w, b, ws, np.zeros(n, np.int32), 0.05, zero, 0.6, 4)
+        xd = dev(torch, x)
+        assert np.array_equal(ctx.qlinear_device(weight, xd, 0.05, zero, 0.6, 4).cpu().numpy(), want)
+        off = torch.empty(rows * k + 1, dtype=xd.dtype, device="cuda")
+        off[1:] = xd.flatten()
+        assert np.array_equal(ctx.qlinear_device(weight, off[1:].view(rows, k), 0.05, zero, 0.6, 4).cpu().numpy(), want)
+        if not in_u8:
+            # one buffer: the output's rows start where the input does
+            both = torch.zeros(max(rows * k, rows * n), dtype=torch.int8, device="cuda")
+            both[:rows * k] = xd.flatten()
+            xin = both[:rows * k].view(rows, k)
+            out = both[:rows * n].view(rows, n)
+            w8a8._check(ctx._L.vxb_qlinear_device(ctx.handle, weight.handle, w8a8._ptr(xin), rows, 0.05, zero, 0.6, 4,
+                                                  w8a8.DT_I8, w8a8.DT_I8, w8a8._ptr(out), n, 0))
+            assert np.array_equal(out.cpu().numpy(), want)
+    weight.close()
+
+
+@pytest.mark.parametrize("scale", [1e-12, 3e-9, 0.0371, 1.9999999, 5e8, 3e9])
+@pytest.mark.parametrize("unsigned,zero", [(False, 0), (False, -128), (True, 255), (True, 3)])
+def test_quantize_linear_scales_and_extremes(torch, ctx, oracle, scale, unsigned, zero):
+    """Scales on both sides of the fast division's range (and the all-ones significand just below 2), ties, the
+    largest and smallest magnitudes, infinities and NaN."""
+    s = np.float32(scale)
+    ties = (np.arange(-600, 600, dtype=np.float32) * np.float32(0.5) * s).astype(np.float32)
+    near = np.concatenate([np.nextafter(ties, np.float32(np.inf)), np.nextafter(ties, np.float32(-np.inf))])
+    ext = np.array([0.0, -0.0, 1e-45, -1e-45, 1e-38, 3.4e38, -3.4e38, np.inf, -np.inf, np.nan, 4096, -4097, 1e20], np.float32)
+    x = np.tile(np.concatenate([ties, near, ext, ext * s]), 4)
+    got = ctx.quantize_linear(dev(torch, x), float(s), zero, unsigned).cpu().numpy()
+    assert np.array_equal(got, oracle.quantize_linear(x, float(s), zero, unsigned))
+
+
 @pytest.mark.parametrize("rows,k", [(1, 64), (5, 1000), (64, 1024), (700, 576), (40, 9000)])
 def test_rmsnorm_products_near_and_far_from_one(torch, ctx, rows, k):
     """The normalized rows against the same arithmetic in 64 bits: ordinary rows, rows scaled to 1e-25 and 1e25 (the

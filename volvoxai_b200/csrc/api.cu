@@ -64,12 +64,13 @@ EncodeTiledFn encode_fn() {
     return g_encode;
 }
 
-// int8 matrix [rows, kpad] row-major -> 2-D tensor map with a (128 B x box_rows) box, 128B swizzle
-bool encode_i8_rows(CUtensorMap* map, const void* base, uint32_t rows, uint32_t kpad, uint32_t box_rows) {
+// int8 matrix [rows, width] row-major, rows one after the other -> 2-D tensor map with a (128 B x box_rows) box,
+// 128B swizzle.  The width is a multiple of 16; the box that crosses a row's end is filled with zeros there.
+bool encode_i8_rows(CUtensorMap* map, const void* base, uint32_t rows, uint32_t width, uint32_t box_rows) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) return false;
-    cuuint64_t dims[2] = {kpad, rows};
-    cuuint64_t strides[1] = {kpad};
+    cuuint64_t dims[2] = {width, rows};
+    cuuint64_t strides[1] = {width};
     cuuint32_t box[2] = {kKAlign, box_rows};
     cuuint32_t elem[2] = {1, 1};
     return fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, elem,
@@ -151,7 +152,7 @@ struct VxbContext {
     int device = 0;
     cudaStream_t stream = nullptr;
     int sm_count = 0;
-    Buffer q, row_scales, bias_eff, stage_in, stage_out;
+    Buffer q, row_scales, stage_in, stage_out;
     Buffer splitk_ws, splitk_counters;   // zero between calls (the decode kernel cleans up)
     int* status = nullptr;        // device block: [0] raised by bounded waits, [1] wait limit in 1024-clock units (0 = default)
     unsigned long long* trace = nullptr;   // caller's device buffer for decode-kernel time stamps, or null
@@ -343,10 +344,11 @@ int launch_decode_fused(VxbContext* ctx, const VxbWeight* w, const float* x, uin
     return 1;
 }
 
-// int32 GEMM + epilogue over already-quantized activations q [rows, kpad].  The kernel is the one
-// vxb_plan() names for this call: the same function tests call without a GPU.
+// int32 GEMM + epilogue over already-quantized activations q [rows, kpad] (q_width: rows of that many bytes, a
+// multiple of 16, in place of kpad; the large-M kernels only).  The kernel is the one vxb_plan() names for this
+// call: the same function tests call without a GPU.
 int run_gemm(VxbContext* ctx, const VxbWeight* w, const int8_t* q, uint32_t rows,
-             const EpilogueParams& epi, int requested, const char* prefix) {
+             const EpilogueParams& epi, int requested, const char* prefix, uint32_t q_width = 0) {
     if (!ctx->tcgen05_ready) {
         CUDA_TRY(gemm_tcgen05_prepare(), 0);
         ctx->tcgen05_ready = true;
@@ -437,7 +439,7 @@ int run_gemm(VxbContext* ctx, const VxbWeight* w, const int8_t* q, uint32_t rows
         }
         case VXB_VARIANT_TCGEN05: case VXB_VARIANT_TCGEN05_PAIR: case VXB_VARIANT_TCGEN05_WIDE: {
             GemmTcgen05Args a;
-            if (!encode_i8_rows(&a.tmap_a, q, rows, w->kpad, 128)) return fail(0, "cuTensorMapEncodeTiled failed for activations");
+            if (!encode_i8_rows(&a.tmap_a, q, rows, q_width ? q_width : w->kpad, 128)) return fail(0, "cuTensorMapEncodeTiled failed for activations");
             a.rows = rows; a.n = w->d_out; a.kpad = w->kpad; a.epi = epi; a.status = ctx->status; a.trace = ctx->trace; a.tma_out = 0;
             if (plan.variant == VXB_VARIANT_TCGEN05_PAIR) {
                 a.tmap_b = w->tmap_w128;   // each CTA of a pair loads half of the tile's weight rows
@@ -647,7 +649,7 @@ void vxb_context_destroy(VxbContext* ctx) {
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     for (auto& v : ctx->prof_events) { for (cudaEvent_t e : v) cudaEventDestroy(e); v.clear(); }
-    ctx->q.release(); ctx->row_scales.release(); ctx->bias_eff.release();
+    ctx->q.release(); ctx->row_scales.release();
     ctx->stage_in.release(); ctx->stage_out.release();
     ctx->splitk_ws.release(); ctx->splitk_counters.release();
     if (ctx->copy_in) {
@@ -1125,22 +1127,33 @@ int vxb_qlinear_device(VxbContext* ctx, const VxbWeight* w, const void* input, u
         return fail(0, "zero point outside its dtype");
     if (!rows) return 1;
     if (ensure_device(ctx) != 1) return -1;
-    // activations into the padded signed layout (U8 -> subtract 128 from codes and zero point)
-    CUDA_TRY(ctx->q.reserve((size_t)rows * w->kpad), 0);
-    CUDA_TRY(ctx->row_scales.reserve((size_t)rows * 4), 0);
-    CUDA_TRY(ctx->bias_eff.reserve((size_t)w->d_out * 4), 0);
-    CUDA_TRY(launch_copy_bytes_padded((const uint8_t*)input, rows, w->d_in, (uint8_t*)ctx->q.ptr, w->kpad,
-                                      in_u8 ? 0x80u : 0u, ctx->stream), -1);
-    CUDA_TRY(launch_fill_f32((float*)ctx->row_scales.ptr, rows, input_scale, ctx->stream), -1);
-    const int32_t signed_zero = in_u8 ? input_zero_point - 128 : input_zero_point;
-    CUDA_TRY(launch_fold_zero_point(w->bias_i32, w->wsum, signed_zero, (int32_t*)ctx->bias_eff.ptr,
-                                    w->d_out, ctx->stream), -1);
-    count_launch(3);
     EpilogueParams epi{};
-    epi.mode = kEpiI8; epi.row_scales = (const float*)ctx->row_scales.ptr; epi.ws = w->ws;
-    epi.bias_i32 = (const int32_t*)ctx->bias_eff.ptr; set_requant_divisor(epi, w, output_scale);
+    epi.mode = kEpiI8; epi.static_scale = input_scale; epi.ws = w->ws;
+    epi.bias_i32 = w->bias_i32; set_requant_divisor(epi, w, output_scale);
+    epi.in_zero = in_u8 ? input_zero_point - 128 : input_zero_point;   // U8 codes are moved to the signed domain below
+    epi.wsum = epi.in_zero ? w->wsum : nullptr;
     epi.out_zero = output_zero_point; epi.out_lo = out_u8 ? 0 : -128; epi.out_hi = out_u8 ? 255 : 127;
     epi.out = output; epi.ld = ldy;
+    // Signed codes are read where they are when a tensor map can describe them (whole 16-byte pieces) and the chosen
+    // kernel takes rows without padding, and when the output does not lie over them; otherwise (and always for U8)
+    // they go through the padded signed layout first.  With the row scales and the folded bias no longer vectors that
+    // launches of their own fill, 4096 x 576 -> 1536 -> 576 between float operators is 6 launches instead of 11 and
+    // 40 us of GPU time instead of 65.
+    const uintptr_t in0 = (uintptr_t)input, in1 = in0 + (size_t)rows * w->d_in;
+    const uintptr_t out0 = (uintptr_t)output, out1 = out0 + (size_t)(rows - 1) * ldy + w->d_out;
+    bool in_place = !in_u8 && (in0 & 15u) == 0 && (w->d_in & 15u) == 0 && (in1 <= out0 || out1 <= in0);
+    if (in_place && w->d_in != w->kpad) {
+        const VxbPlanQuery query = plan_query(ctx, w, rows, epi, route, false);
+        VxbLaunchPlan plan;
+        char why[160];
+        in_place = vxb_plan(&query, &plan, why, sizeof why) == 1 &&
+                   (plan.variant == VXB_VARIANT_TCGEN05 || plan.variant == VXB_VARIANT_TCGEN05_PAIR);
+    }
+    if (in_place) return run_gemm(ctx, w, (const int8_t*)input, rows, epi, route, "static+", w->d_in);
+    CUDA_TRY(ctx->q.reserve((size_t)rows * w->kpad), 0);
+    CUDA_TRY(launch_copy_bytes_padded((const uint8_t*)input, rows, w->d_in, (uint8_t*)ctx->q.ptr, w->kpad,
+                                      in_u8 ? 0x80u : 0u, ctx->stream), -1);
+    count_launch();
     return run_gemm(ctx, w, (const int8_t*)ctx->q.ptr, rows, epi, route, "static+");
 }
 

@@ -1,6 +1,9 @@
 // The F32 <-> byte boundary of a static W8A8 island and the byte-to-byte bridge between two
 // quantized domains: QuantizeLinear, DequantizeLinear, RequantizeLinear. HBM-bound elementwise
-// work: 16 elements per thread, 128-bit accesses where the pointers allow.
+// work: 16 elements per thread, 128-bit accesses where the pointers allow.  Between fp32 and bytes a thread's
+// elements are four groups of four, 1024 elements apart, so that a warp's load or store of either side is one run
+// of consecutive bytes (sixteen consecutive elements per thread were 64-byte strides on the fp32 side).  All
+// three are launched with programmatic dependent launch, each in the shadow of the launch before it.
 //
 // Arithmetic (CPU authority of the reference, restated in oracle/w8a8_oracle.c):
 //   quantize    NaN -> zero point; t = f32(x / scale) + f32(zero); saturate; ties to even
@@ -12,6 +15,7 @@
 // vx_cuda_requantize_i8u8 (native/src/backends/cuda/kernels/
 // cuda_forward_quantized_basic_kernels.inc:163-193), one element per thread.
 #include "common.cuh"
+#include <string.h>
 
 namespace vxb {
 
@@ -19,14 +23,6 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kPerThread = 16;
-
-__device__ __forceinline__ int32_t load_byte(const uint8_t* p, bool is_unsigned) {
-    return is_unsigned ? (int32_t)*p : (int32_t)*reinterpret_cast<const int8_t*>(p);
-}
-__device__ __forceinline__ int32_t byte_of(uint32_t word, int i, bool is_unsigned) {
-    const uint32_t b = (word >> (8 * i)) & 0xffu;
-    return is_unsigned ? (int32_t)b : (int32_t)(int8_t)b;
-}
 
 __device__ __forceinline__ int32_t quantize1(float v, float scale, float zero_f, int32_t zero, float lo_f,
                                              float hi_f, int32_t lo, int32_t hi) {
@@ -36,84 +32,110 @@ __device__ __forceinline__ int32_t quantize1(float v, float scale, float zero_f,
     if (t >= hi_f) return hi;
     return __float2int_rn(t);   // finite and inside the range here: round to nearest even
 }
-__device__ __forceinline__ int32_t requantize1(int32_t x, int32_t in_zero, float multiplier, float zero_f,
-                                               int32_t zero, float lo_f, float hi_f, int32_t lo, int32_t hi) {
-    const float t = __fadd_rn(__fmul_rn(__int2float_rn(x - in_zero), multiplier), zero_f);
-    if (t != t) return zero;
-    if (t <= lo_f) return lo;
-    if (t >= hi_f) return hi;
-    return __float2int_rn(t);
+// f32(byte - zero) without a conversion instruction: the byte in the low mantissa bits of 2^23, less 2^23 + zero (and
+// 128 more for signed bytes, whose sign bit is flipped first).  Every step is exact.
+__device__ __forceinline__ float centred(uint32_t word, int i, float base) {
+    return __fadd_rn(__uint_as_float(__byte_perm(word, 0x4B000000u, 0x7440 | i)), -base);
+}
+__device__ __forceinline__ float centre_base(int32_t zero, bool is_unsigned) {
+    return 8388608.0f + __int2float_rn(zero + (is_unsigned ? 0 : 128));
+}
+// one rounding per step; the product can be infinite (it then saturates), never NaN
+__device__ __forceinline__ float requantized(float x, float multiplier, float zero_f) { return __fadd_rn(__fmul_rn(x, multiplier), zero_f); }
+
+// FAST (the host found the scale within 2^+-30 and its significand not all ones): the IEEE quotient through
+// div_const.  Elements whose quotient is far outside every byte range are first brought to +-4096 scales, which
+// saturates all the same and keeps div_const's operands in its range; a quotient too small for it rounds, with the
+// zero point added, to the zero point either way.
+template <bool FAST, bool UNSIGNED>
+__device__ __forceinline__ int32_t quantize_any(float v, float scale, float rcp, float bound, float zero_f, int32_t zero) {
+    if constexpr (FAST) {
+        const float t = __fadd_rn(div_const(fminf(fmaxf(v, -bound), bound), scale, rcp), zero_f);
+        return v != v ? zero : byte_code<UNSIGNED>(t);
+    } else {
+        constexpr int32_t lo = UNSIGNED ? 0 : -128, hi = UNSIGNED ? 255 : 127;
+        return quantize1(v, scale, zero_f, zero, (float)lo, (float)hi, lo, hi);
+    }
 }
 
+template <bool FAST, bool UNSIGNED>
 __global__ void __launch_bounds__(kThreads)
-quantize_linear_kernel(const float* __restrict__ x, unsigned long long n, float scale, int32_t zero, int32_t lo,
-                       int32_t hi, uint8_t* __restrict__ out, int vec) {
-    const float zero_f = __int2float_rn(zero), lo_f = __int2float_rn(lo), hi_f = __int2float_rn(hi);
-    const unsigned long long base = ((unsigned long long)blockIdx.x * kThreads + threadIdx.x) * kPerThread;
-    if (base >= n) return;
-    if (vec && base + kPerThread <= n) {
-        uint32_t w[4];
+quantize_linear_kernel(const float* __restrict__ x, unsigned long long n, float scale, float rcp, int32_t zero,
+                       uint8_t* __restrict__ out, int vec) {
+    pdl_release();
+    pdl_wait();
+    const float zero_f = __int2float_rn(zero), bound = __fmul_rn(scale, 4096.0f);
+    const unsigned long long block = (unsigned long long)blockIdx.x * (kThreads * kPerThread);
+    if (vec && block + kThreads * kPerThread <= n) {
+        const float4* in = reinterpret_cast<const float4*>(x + block) + threadIdx.x;
+        uint32_t* dst = reinterpret_cast<uint32_t*>(out + block) + threadIdx.x;
+        float4 v[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) v[j] = __ldg(in + j * kThreads);
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            const float4 v = __ldg(reinterpret_cast<const float4*>(x + base) + j);
-            const int32_t a = quantize1(v.x, scale, zero_f, zero, lo_f, hi_f, lo, hi);
-            const int32_t b = quantize1(v.y, scale, zero_f, zero, lo_f, hi_f, lo, hi);
-            const int32_t c = quantize1(v.z, scale, zero_f, zero, lo_f, hi_f, lo, hi);
-            const int32_t d = quantize1(v.w, scale, zero_f, zero, lo_f, hi_f, lo, hi);
-            w[j] = __byte_perm(__byte_perm(a, b, 0x0040), __byte_perm(c, d, 0x0040), 0x5410);
+            const int32_t a = quantize_any<FAST, UNSIGNED>(v[j].x, scale, rcp, bound, zero_f, zero);
+            const int32_t b = quantize_any<FAST, UNSIGNED>(v[j].y, scale, rcp, bound, zero_f, zero);
+            const int32_t c = quantize_any<FAST, UNSIGNED>(v[j].z, scale, rcp, bound, zero_f, zero);
+            const int32_t d = quantize_any<FAST, UNSIGNED>(v[j].w, scale, rcp, bound, zero_f, zero);
+            dst[j * kThreads] = __byte_perm(__byte_perm(a, b, 0x0040), __byte_perm(c, d, 0x0040), 0x5410);
         }
-        *reinterpret_cast<uint4*>(out + base) = make_uint4(w[0], w[1], w[2], w[3]);
     } else {
-        for (unsigned long long i = base; i < n && i < base + kPerThread; i++)
-            out[i] = (uint8_t)quantize1(x[i], scale, zero_f, zero, lo_f, hi_f, lo, hi);
+        for (unsigned long long i = block + threadIdx.x; i < n && i < block + kThreads * kPerThread; i += kThreads)
+            out[i] = (uint8_t)quantize_any<FAST, UNSIGNED>(x[i], scale, rcp, bound, zero_f, zero);
     }
 }
 
 __global__ void __launch_bounds__(kThreads)
 dequantize_linear_kernel(const uint8_t* __restrict__ x, unsigned long long n, float scale, int32_t zero,
                          int is_unsigned, float* __restrict__ out, int vec) {
-    const unsigned long long base = ((unsigned long long)blockIdx.x * kThreads + threadIdx.x) * kPerThread;
-    if (base >= n) return;
-    if (vec && base + kPerThread <= n) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(x + base));
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    pdl_release();
+    pdl_wait();
+    const float base = centre_base(zero, is_unsigned);
+    const uint32_t flip = is_unsigned ? 0u : 0x80808080u;
+    const unsigned long long block = (unsigned long long)blockIdx.x * (kThreads * kPerThread);
+    if (vec && block + kThreads * kPerThread <= n) {
+        const uint32_t* in = reinterpret_cast<const uint32_t*>(x + block) + threadIdx.x;
+        float4* dst = reinterpret_cast<float4*>(out + block) + threadIdx.x;
+        uint32_t w[4];
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            float4 o;
-            o.x = __fmul_rn(__int2float_rn(byte_of(w[j], 0, is_unsigned) - zero), scale);
-            o.y = __fmul_rn(__int2float_rn(byte_of(w[j], 1, is_unsigned) - zero), scale);
-            o.z = __fmul_rn(__int2float_rn(byte_of(w[j], 2, is_unsigned) - zero), scale);
-            o.w = __fmul_rn(__int2float_rn(byte_of(w[j], 3, is_unsigned) - zero), scale);
-            reinterpret_cast<float4*>(out + base)[j] = o;
-        }
+        for (int j = 0; j < 4; j++) w[j] = __ldg(in + j * kThreads) ^ flip;
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            dst[j * kThreads] = make_float4(__fmul_rn(centred(w[j], 0, base), scale), __fmul_rn(centred(w[j], 1, base), scale),
+                                            __fmul_rn(centred(w[j], 2, base), scale), __fmul_rn(centred(w[j], 3, base), scale));
     } else {
-        for (unsigned long long i = base; i < n && i < base + kPerThread; i++)
-            out[i] = __fmul_rn(__int2float_rn(load_byte(x + i, is_unsigned) - zero), scale);
+        for (unsigned long long i = block + threadIdx.x; i < n && i < block + kThreads * kPerThread; i += kThreads)
+            out[i] = __fmul_rn(centred(x[i] ^ (flip & 0xffu), 0, base), scale);
     }
 }
 
+template <bool OUT_UNSIGNED>
 __global__ void __launch_bounds__(kThreads)
 requantize_linear_kernel(const uint8_t* __restrict__ x, unsigned long long n, float multiplier, int32_t in_zero,
-                         int in_unsigned, int32_t zero, int32_t lo, int32_t hi, uint8_t* __restrict__ out, int vec) {
-    const float zero_f = __int2float_rn(zero), lo_f = __int2float_rn(lo), hi_f = __int2float_rn(hi);
-    const unsigned long long base = ((unsigned long long)blockIdx.x * kThreads + threadIdx.x) * kPerThread;
-    if (base >= n) return;
-    if (vec && base + kPerThread <= n) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(x + base));
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+                         int in_unsigned, int32_t zero, uint8_t* __restrict__ out, int vec) {
+    pdl_release();
+    pdl_wait();
+    const float base = centre_base(in_zero, in_unsigned), zero_f = __int2float_rn(zero);
+    const uint32_t flip = in_unsigned ? 0u : 0x80808080u;
+    const unsigned long long at = ((unsigned long long)blockIdx.x * kThreads + threadIdx.x) * kPerThread;
+    if (at >= n) return;
+    if (vec && at + kPerThread <= n) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(x + at));
+        const uint32_t w[4] = {v.x ^ flip, v.y ^ flip, v.z ^ flip, v.w ^ flip};
         uint32_t o[4];
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            const int32_t a = requantize1(byte_of(w[j], 0, in_unsigned), in_zero, multiplier, zero_f, zero, lo_f, hi_f, lo, hi);
-            const int32_t b = requantize1(byte_of(w[j], 1, in_unsigned), in_zero, multiplier, zero_f, zero, lo_f, hi_f, lo, hi);
-            const int32_t c = requantize1(byte_of(w[j], 2, in_unsigned), in_zero, multiplier, zero_f, zero, lo_f, hi_f, lo, hi);
-            const int32_t d = requantize1(byte_of(w[j], 3, in_unsigned), in_zero, multiplier, zero_f, zero, lo_f, hi_f, lo, hi);
+            const int32_t a = byte_code<OUT_UNSIGNED>(requantized(centred(w[j], 0, base), multiplier, zero_f));
+            const int32_t b = byte_code<OUT_UNSIGNED>(requantized(centred(w[j], 1, base), multiplier, zero_f));
+            const int32_t c = byte_code<OUT_UNSIGNED>(requantized(centred(w[j], 2, base), multiplier, zero_f));
+            const int32_t d = byte_code<OUT_UNSIGNED>(requantized(centred(w[j], 3, base), multiplier, zero_f));
             o[j] = __byte_perm(__byte_perm(a, b, 0x0040), __byte_perm(c, d, 0x0040), 0x5410);
         }
-        *reinterpret_cast<uint4*>(out + base) = make_uint4(o[0], o[1], o[2], o[3]);
+        *reinterpret_cast<uint4*>(out + at) = make_uint4(o[0], o[1], o[2], o[3]);
     } else {
-        for (unsigned long long i = base; i < n && i < base + kPerThread; i++)
-            out[i] = (uint8_t)requantize1(load_byte(x + i, in_unsigned), in_zero, multiplier, zero_f, zero, lo_f, hi_f, lo, hi);
+        for (unsigned long long i = at; i < n && i < at + kPerThread; i++)
+            out[i] = (uint8_t)byte_code<OUT_UNSIGNED>(requantized(centred(x[i] ^ (flip & 0xffu), 0, base), multiplier, zero_f));
     }
 }
 
@@ -127,27 +149,28 @@ inline int aligned16(const void* a, const void* b) { return (((uintptr_t)a | (ui
 cudaError_t launch_quantize_linear(const float* x, unsigned long long n, float scale, int32_t zero, bool out_unsigned,
                                    void* out, cudaStream_t stream) {
     if (!n) return cudaSuccess;
-    quantize_linear_kernel<<<grid_for(n), kThreads, 0, stream>>>(x, n, scale, zero, out_unsigned ? 0 : -128,
-                                                                out_unsigned ? 255 : 127, (uint8_t*)out, aligned16(x, out));
-    return cudaGetLastError();
+    uint32_t bits;
+    memcpy(&bits, &scale, 4);
+    const bool fast = scale >= 9.31322574615478515625e-10f && scale <= 1073741824.0f && (bits & 0x007fffffu) != 0x007fffffu;
+    auto kernel = fast ? (out_unsigned ? quantize_linear_kernel<true, true> : quantize_linear_kernel<true, false>)
+                       : (out_unsigned ? quantize_linear_kernel<false, true> : quantize_linear_kernel<false, false>);
+    return launch_pdl(kernel, dim3(grid_for(n)), dim3(kThreads), 0, stream, x, n, scale, (float)(1.0 / (double)scale), zero,
+                      (uint8_t*)out, aligned16(x, out));
 }
 
 cudaError_t launch_dequantize_linear(const void* x, unsigned long long n, float scale, int32_t zero, bool in_unsigned,
                                      float* out, cudaStream_t stream) {
     if (!n) return cudaSuccess;
-    dequantize_linear_kernel<<<grid_for(n), kThreads, 0, stream>>>((const uint8_t*)x, n, scale, zero, in_unsigned ? 1 : 0,
-                                                                  out, aligned16(x, out));
-    return cudaGetLastError();
+    return launch_pdl(dequantize_linear_kernel, dim3(grid_for(n)), dim3(kThreads), 0, stream, (const uint8_t*)x, n, scale, zero,
+                      in_unsigned ? 1 : 0, out, aligned16(x, out));
 }
 
 cudaError_t launch_requantize_linear(const void* x, unsigned long long n, float multiplier, int32_t in_zero,
                                      bool in_unsigned, int32_t out_zero, bool out_unsigned, void* out,
                                      cudaStream_t stream) {
     if (!n) return cudaSuccess;
-    requantize_linear_kernel<<<grid_for(n), kThreads, 0, stream>>>((const uint8_t*)x, n, multiplier, in_zero,
-                                                                  in_unsigned ? 1 : 0, out_zero, out_unsigned ? 0 : -128,
-                                                                  out_unsigned ? 255 : 127, (uint8_t*)out, aligned16(x, out));
-    return cudaGetLastError();
+    return launch_pdl(out_unsigned ? requantize_linear_kernel<true> : requantize_linear_kernel<false>, dim3(grid_for(n)), dim3(kThreads), 0,
+                      stream, (const uint8_t*)x, n, multiplier, in_zero, in_unsigned ? 1 : 0, out_zero, (uint8_t*)out, aligned16(x, out));
 }
 
 }  // namespace vxb

@@ -20,10 +20,13 @@ enum Epilogue : int { kEpiAcc = 0, kEpiF32 = 1, kEpiI8 = 2 };
 
 struct EpilogueParams {
     int mode;                 // Epilogue
-    const float* row_scales;  // [rows]   activation scale per token (NaN = invalid row)
+    const float* row_scales;  // [rows]   activation scale per token (NaN = invalid row), or null:
+    float static_scale;       //          one scale for all rows (static activations)
     const float* ws;          // [N]      weight scale per output channel
     const float* bias_f32;    // [N] or nullptr (E1)
-    const int32_t* bias_i32;  // [N] or nullptr (E2, accumulator domain, zero-point folded)
+    const int32_t* bias_i32;  // [N] or nullptr (E2, accumulator domain)
+    const int32_t* wsum;      // [N] code sums, or nullptr: the activations have a zero point in_zero, which leaves
+    int32_t in_zero;          // in_zero * wsum[n] to be taken off the bias
     float out_scale;          // E2
     float out_rcp;            // E2: RN(1/out_scale), used when fast_div != 0
     int32_t fast_div;         // E2: host verified that division by out_scale may use div_const()
@@ -157,6 +160,15 @@ __device__ __forceinline__ int32_t epi_i8_sat(int32_t acc, float as, float ws, f
     return q;
 }
 
+// Round to nearest even and saturate to the byte range, the code in the low byte: clamp, then let the addition of
+// 1.5 * 2^23 do the rounding.  Three instructions of the wide pipes instead of one conversion; a conversion runs on
+// the XU pipe at 16 per clock and SM, and the accumulator's int32 -> fp32 already takes one there per output.
+// Not for NaN.
+template <bool UNSIGNED>
+__device__ __forceinline__ int32_t byte_code(float v) {
+    return __float_as_int(__fadd_rn(fminf(fmaxf(v, UNSIGNED ? 0.0f : -128.0f), UNSIGNED ? 255.0f : 127.0f), 12582912.0f));
+}
+
 // The same two elements at a time with the packed fp32 instructions of sm_100 (mul/fma.rn.f32x2:
 // each half rounded to nearest like the scalar instruction, subnormals kept), which halves the
 // floating-point instruction count of the requantization. A pair lives in a 64-bit register.
@@ -200,13 +212,8 @@ __device__ __forceinline__ void epi_i8_sat2(int32_t acc0, int32_t acc1, uint64_t
     // the zero point is added with scalar instructions: a packed add right after the packed
     // multiply came out as one fused multiply-add (33.4999962 instead of 33.5 in a tie case)
     if (ADD_ZERO) { m0 = __fadd_rn(m0, c.zero); m1 = __fadd_rn(m1, c.zero); }
-    if (UNSIGNED) {
-        asm("cvt.rni.sat.u8.f32 %0, %1;" : "=r"(q0) : "f"(m0));
-        asm("cvt.rni.sat.u8.f32 %0, %1;" : "=r"(q1) : "f"(m1));
-    } else {
-        asm("cvt.rni.sat.s8.f32 %0, %1;" : "=r"(q0) : "f"(m0));
-        asm("cvt.rni.sat.s8.f32 %0, %1;" : "=r"(q1) : "f"(m1));
-    }
+    q0 = byte_code<UNSIGNED>(m0);
+    q1 = byte_code<UNSIGNED>(m1);
 }
 
 // E1 for two neighbouring channels: (f32(acc) * (as * ws)) + bias, each step rounded; the two
@@ -228,6 +235,16 @@ __device__ __forceinline__ float epi_silu_mul(float gate, float up) {
     return __fmul_rn(__fmul_rn(gate, sig), up);
 }
 
+// The row's activation scale, and the channel's int32 bias with the activations' zero point folded in (the same
+// wrapping integers as a folded bias vector, without a launch that makes one).
+__device__ __forceinline__ float epi_row_scale(const EpilogueParams& p, uint32_t row) {
+    return p.row_scales ? __ldg(p.row_scales + row) : p.static_scale;
+}
+__device__ __forceinline__ int32_t epi_bias_i32(const EpilogueParams& p, uint32_t n) {
+    const uint32_t b = p.bias_i32 ? (uint32_t)__ldg(p.bias_i32 + n) : 0u;
+    return (int32_t)(p.wsum ? b - (uint32_t)p.in_zero * (uint32_t)__ldg(p.wsum + n) : b);
+}
+
 // One output element through the selected epilogue (scalar path).
 __device__ __forceinline__ void epi_store(const EpilogueParams& p, uint32_t row, uint32_t col,
                                           int32_t acc) {
@@ -235,11 +252,11 @@ __device__ __forceinline__ void epi_store(const EpilogueParams& p, uint32_t row,
     if (p.mode == kEpiAcc) {
         ((int32_t*)p.out)[at] = acc;
     } else if (p.mode == kEpiF32) {
-        ((float*)p.out)[at] = epi_f32(acc, p.row_scales[row], p.ws[col],
+        ((float*)p.out)[at] = epi_f32(acc, epi_row_scale(p, row), p.ws[col],
                                       p.bias_f32 ? p.bias_f32[col] : 0.0f);
     } else {
-        const int32_t a = acc + (p.bias_i32 ? p.bias_i32[col] : 0);
-        ((int8_t*)p.out)[at] = (int8_t)epi_i8(a, p.row_scales[row], p.ws[col], p.out_scale,
+        const int32_t a = acc + epi_bias_i32(p, col);
+        ((int8_t*)p.out)[at] = (int8_t)epi_i8(a, epi_row_scale(p, row), p.ws[col], p.out_scale,
                                               p.out_zero, p.out_lo, p.out_hi);
     }
 }
@@ -286,14 +303,7 @@ cudaError_t launch_quantize_rows(const float* x, uint32_t rows, uint32_t k, int8
 uint32_t quantize_vec_threads(uint32_t rows, uint32_t k);   // threads per row of the quantizers with 128-bit loads
 uint32_t quantize_any_threads(uint32_t rows, uint32_t k);   // threads per row of the quantizer that takes any width and alignment
 
-// Fill a float array with one value (static-activation QLinear row scales).
-cudaError_t launch_fill_f32(float* dst, uint32_t count, float value, cudaStream_t stream);
-
-// bias_eff[n] = bias[n] - input_zero * wsum[n]  (activation zero-point folding)
-cudaError_t launch_fold_zero_point(const int32_t* bias, const int32_t* wsum, int32_t input_zero,
-                                   int32_t* out, uint32_t n, cudaStream_t stream);
-
-// Convert U8 activations to the signed domain (x ^ 0x80) with row padding.
+// Activation bytes into the padded row layout, with U8 codes converted to the signed domain (x ^ 0x80).
 cudaError_t launch_copy_bytes_padded(const uint8_t* src, uint32_t rows, uint32_t k, uint8_t* dst,
                                      uint32_t ld, uint32_t xor_mask, cudaStream_t stream);
 

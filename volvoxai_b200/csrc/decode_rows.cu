@@ -498,14 +498,14 @@ decode_rows_kernel(const __grid_constant__ DecodeRowsArgs args) {
                 if (n < args.n && ep.mode != kEpiAcc) {
                     wsv = __ldg(ep.ws + n);
                     if (ep.mode == kEpiF32) bv = ep.bias_f32 ? __ldg(ep.bias_f32 + n) : 0.0f;
-                    else bv = __int_as_float(ep.bias_i32 ? __ldg(ep.bias_i32 + n) : 0);
+                    else bv = __int_as_float(epi_bias_i32(ep, n));
                 }
                 s_ws[i] = wsv; s_bias[i] = bv;
             }
             if (t == 0) {
                 // from here on: reads of what the preceding kernel wrote, writes of what it may read
                 pdl_wait();
-                if (e < 128 && !fused) s_as[e] = (e < args.rows && ep.mode != kEpiAcc) ? __ldg(ep.row_scales + e) : 0.0f;
+                if (e < 128 && !fused) s_as[e] = (e < args.rows && ep.mode != kEpiAcc) ? epi_row_scale(ep, e) : 0.0f;
             }
             if constexpr (Cfg::kParkAll) {
                 if (tiles == 1) break;   // the single tile is drained by every warp of the CTA, below

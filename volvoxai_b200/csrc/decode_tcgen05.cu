@@ -187,7 +187,7 @@ decode_i8_tcgen05_kernel(const __grid_constant__ DecodeTcgen05Args args) {
         const float lo_f = __int2float_rn(ep.out_lo), hi_f = __int2float_rn(ep.out_hi);
         // everything below reads what the preceding kernel wrote, or writes what it may read
         pdl_wait();
-        if (e < MT) s_as[e] = (e < args.rows && ep.mode != kEpiAcc) ? __ldg(ep.row_scales + e) : 0.0f;
+        if (e < MT) s_as[e] = (e < args.rows && ep.mode != kEpiAcc) ? epi_row_scale(ep, e) : 0.0f;
         epi_bar();
 
         // One 32-token chunk of channel n through the selected epilogue.
@@ -215,7 +215,7 @@ decode_i8_tcgen05_kernel(const __grid_constant__ DecodeTcgen05Args args) {
             const bool n_ok = n < args.n;
             wsv = (n_ok && ep.mode != kEpiAcc) ? __ldg(ep.ws + n) : 0.0f;
             bias_f = (n_ok && ep.mode == kEpiF32 && ep.bias_f32) ? __ldg(ep.bias_f32 + n) : 0.0f;
-            bias_i = (n_ok && ep.mode == kEpiI8 && ep.bias_i32) ? __ldg(ep.bias_i32 + n) : 0;
+            bias_i = (n_ok && ep.mode == kEpiI8) ? epi_bias_i32(ep, n) : 0;
         };
 
         // A contiguous unit range holds at most two partial segments (its first and its last);

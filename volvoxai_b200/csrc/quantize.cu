@@ -279,22 +279,31 @@ quantize_rows_any(const float* __restrict__ x, uint32_t rows, uint32_t k, int8_t
         out[j] = (j < k && !bad) ? (int8_t)(div.fast ? quant1<true>(__ldg(in + j), div) : quant1<false>(__ldg(in + j), div)) : (int8_t)0;
 }
 
-__global__ void fill_f32_kernel(float* dst, uint32_t count, float value) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < count) dst[i] = value;
-}
-
-__global__ void fold_zero_point_kernel(const int32_t* bias, const int32_t* wsum, int32_t zero,
-                                       int32_t* out, uint32_t n) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = (bias ? bias[i] : 0) - zero * wsum[i];
-}
-
-__global__ void copy_bytes_padded_kernel(const uint8_t* __restrict__ src, uint32_t rows, uint32_t k,
-                                         uint8_t* __restrict__ dst, uint32_t ld, uint32_t xor_mask) {
-    const uint32_t row = blockIdx.y;
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < ld; j += gridDim.x * blockDim.x)
-        dst[(size_t)row * ld + j] = j < k ? (uint8_t)(src[(size_t)row * k + j] ^ xor_mask) : (uint8_t)0;
+// Sixteen output bytes per thread; VEC: rows of whole 16-byte pieces, read as such.
+template <bool VEC>
+__global__ void __launch_bounds__(kThreads)
+copy_bytes_padded_kernel(const uint8_t* __restrict__ src, uint32_t rows, uint32_t k, uint8_t* __restrict__ dst,
+                         uint32_t ld, uint32_t xor_mask) {
+    pdl_release();
+    pdl_wait();
+    const uint32_t per_row = ld / 16u;
+    const uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
+    const uint32_t row = (uint32_t)(i / per_row), at = (uint32_t)(i - (uint64_t)row * per_row) * 16u;
+    if (row >= rows) return;
+    const uint8_t* in = src + (size_t)row * k + at;
+    uint32_t w[4] = {0u, 0u, 0u, 0u};
+    if constexpr (VEC) {
+        if (at < k) {
+            const uint4 v = __ldg(reinterpret_cast<const uint4*>(in));
+            const uint32_t m = xor_mask * 0x01010101u;
+            w[0] = v.x ^ m; w[1] = v.y ^ m; w[2] = v.z ^ m; w[3] = v.w ^ m;
+        }
+    } else {
+#pragma unroll
+        for (uint32_t j = 0; j < 16; j++)
+            if (at + j < k) w[j >> 2] |= (uint32_t)(uint8_t)(__ldg(in + j) ^ xor_mask) << (8u * (j & 3u));
+    }
+    *reinterpret_cast<uint4*>(dst + (size_t)row * ld + at) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
 // One warp per weight row: copy (with optional ^0x80), zero the padding, sum the codes.
@@ -587,31 +596,14 @@ cudaError_t launch_rmsnorm_quantize_rows(const float* x, const float* gamma, flo
     }
 }
 
-cudaError_t launch_fill_f32(float* dst, uint32_t count, float value, cudaStream_t stream) {
-    if (!count) return cudaSuccess;
-    fill_f32_kernel<<<(count + 255) / 256, 256, 0, stream>>>(dst, count, value);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_fold_zero_point(const int32_t* bias, const int32_t* wsum, int32_t input_zero,
-                                   int32_t* out, uint32_t n, cudaStream_t stream) {
-    if (!n) return cudaSuccess;
-    fold_zero_point_kernel<<<(n + 255) / 256, 256, 0, stream>>>(bias, wsum, input_zero, out, n);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_copy_bytes_padded(const uint8_t* src, uint32_t rows, uint32_t k, uint8_t* dst,
                                      uint32_t ld, uint32_t xor_mask, cudaStream_t stream) {
     if (!rows) return cudaSuccess;
-    dim3 grid((ld + 1023) / 1024 < 8 ? (ld + 1023) / 1024 : 8, rows);
-    // grid.y is limited to 65535: larger row counts go in slabs
-    for (uint32_t r0 = 0; r0 < rows; r0 += 65535u) {
-        const uint32_t cnt = rows - r0 < 65535u ? rows - r0 : 65535u;
-        grid.y = cnt;
-        copy_bytes_padded_kernel<<<grid, 256, 0, stream>>>(src + (size_t)r0 * k, cnt, k,
-                                                            dst + (size_t)r0 * ld, ld, xor_mask);
-    }
-    return cudaGetLastError();
+    if (ld % 16u || ((uintptr_t)dst & 15u)) return cudaErrorInvalidValue;
+    const uint32_t grid = (uint32_t)(((uint64_t)rows * (ld / 16u) + kThreads - 1) / kThreads);
+    if (k % 16u == 0 && ((uintptr_t)src & 15u) == 0)
+        return launch_pdl(copy_bytes_padded_kernel<true>, dim3(grid), dim3(kThreads), 0, stream, src, rows, k, dst, ld, xor_mask);
+    return launch_pdl(copy_bytes_padded_kernel<false>, dim3(grid), dim3(kThreads), 0, stream, src, rows, k, dst, ld, xor_mask);
 }
 
 cudaError_t launch_repack_weight(const uint8_t* src, uint32_t src_ld, uint32_t n, uint32_t k,
