@@ -128,6 +128,34 @@ def test_quantize_linear_scales_and_extremes(torch, ctx, oracle, scale, unsigned
     assert np.array_equal(got, oracle.quantize_linear(x, float(s), zero, unsigned))
 
 
+@pytest.mark.parametrize("group", [32, 64, 128, 256])
+@pytest.mark.parametrize("rows,k,n", [(5, 300, 1), (8, 640, 129), (9, 4096, 100), (17, 1283, 300), (33, 896, 64), (64, 2176, 257),
+                                      (7, 272, 10000), (40, 384, 19200)])
+def test_grouped_few_rows(torch, ctx, oracle, group, rows, k, n):
+    """Every token-slot count and both tile heights of the few-row kernel: ragged channels, a last stage half empty, a
+    last group cut short, more tiles than SMs; rows one past a slot count take the next one."""
+    from volvoxai_b200 import _lib, w8a8
+    rng = np.random.default_rng(group + rows * 7 + k + n)
+    w = rng.integers(-127, 128, size=(n, k), dtype=np.int8)
+    words = wl.pack_w8_words(w)
+    gs = rng.uniform(0.001, 0.05, size=(n, (k + group - 1) // group)).astype(np.float32)
+    bias = rng.standard_normal(n).astype(np.float32)
+    x = (rng.standard_normal((rows, k)) * 2).astype(np.float32)
+    x[1] = 0
+    x[2, k // 3] = np.nan
+    wg = w8a8.Weight.from_w8_words(ctx, words, gs, k, group, bias_f32=bias)
+    wide = torch.full((rows, n + 5), 99.0, device="cuda")
+    ctx.linear_f32(wg, dev(torch, x), out=wide[:, 2:2 + n])
+    assert "tcgen05-grouped-i8" in _lib.last_route()
+    got = wide.cpu().numpy()
+    assert (got[:, :2] == 99).all() and (got[:, 2 + n:] == 99).all()
+    y, want = got[:, 2:2 + n], oracle.packed_linear_w8_grouped(x, words, gs, group, bias)
+    assert np.array_equal(np.isnan(y), np.isnan(want))
+    ok = ~np.isnan(want)
+    assert np.array_equal(bits(y[ok]), bits(want[ok]))
+    wg.close()
+
+
 @pytest.mark.parametrize("rows,k", [(1, 64), (5, 1000), (64, 1024), (700, 576), (40, 9000)])
 def test_rmsnorm_products_near_and_far_from_one(torch, ctx, rows, k):
     """The normalized rows against the same arithmetic in 64 bits: ordinary rows, rows scaled to 1e-25 and 1e25 (the

@@ -385,13 +385,18 @@ int run_gemm(VxbContext* ctx, const VxbWeight* w, const int8_t* q, uint32_t rows
                 ctx->grouped_ready = true;
             }
             GemmGroupedArgs a;
-            if (!encode_i8_rows(&a.tmap_a, q, rows, w->kpad, 128)) return fail(0, "cuTensorMapEncodeTiled failed for activations");
-            a.tmap_b = w->tmap_w128;
+            const GroupedFewShape few = grouped_few_shape(rows, w->d_out, ctx->sm_count);
+            if (few.slots ? !(encode_i8_kblocks(&a.tmap_a, q, rows, w->kpad, few.slots, 2) &&
+                              encode_i8_kblocks(&a.tmap_b, w->w, w->d_out, w->kpad, few.channels, 2))
+                          : !encode_i8_rows(&a.tmap_a, q, rows, w->kpad, 128))
+                return fail(0, "cuTensorMapEncodeTiled failed for activations");
+            if (!few.slots) a.tmap_b = w->tmap_w128;
             a.rows = rows; a.n = w->d_out; a.kpad = w->kpad;
             a.group = w->group; a.groups = w->groups; a.n_pad = w->n_pad; a.gscales_t = w->gscales_t;
             a.row_scales = epi.row_scales; a.bias = epi.bias_f32; a.out = (float*)epi.out; a.ld = epi.ld;
             a.status = ctx->status;
-            LAUNCH_TRY(launch_gemm_grouped_tcgen05(a, ctx->sm_count, ctx->stream));
+            if (few.slots) LAUNCH_TRY(launch_gemm_grouped_few(a, ctx->sm_count, ctx->stream));
+            else LAUNCH_TRY(launch_gemm_grouped_tcgen05(a, ctx->sm_count, ctx->stream));
             break;
         }
         case VXB_VARIANT_DP4A_GROUPED:

@@ -377,6 +377,12 @@ struct GemmGroupedArgs {
 };
 cudaError_t gemm_grouped_tcgen05_prepare();
 cudaError_t launch_gemm_grouped_tcgen05(const GemmGroupedArgs& args, int sm_count, cudaStream_t stream);
+// K2f: the same for up to kGroupedFewMaxRows rows, weights as the M operand; both tensor maps are the 3-D view
+// {128 B, rows, K blocks}, boxes of two K blocks x the shape's token slots (tmap_a) and channels (tmap_b).
+constexpr uint32_t kGroupedFewMaxRows = 64;
+struct GroupedFewShape { uint32_t tokens, slots, channels, grid, threads; };   // live tokens, token columns (0: not served), ...
+GroupedFewShape grouped_few_shape(uint32_t rows, uint32_t n, int sm_count);
+cudaError_t launch_gemm_grouped_few(const GemmGroupedArgs& args, int sm_count, cudaStream_t stream);
 
 // K3: decode kernel in which every CTA owns whole output channels (rows <= 128).
 // tile_rows / tiles_per_cta come from decode_rows_plan(); tmap_w has a box of tile_rows rows,

@@ -103,6 +103,14 @@ bool geometry(VxbVariantId id, const VxbPlanQuery& q, VxbLaunchPlan* p) {
             p->grid = ceil_div(q.n, 128) * (q.rows == 1 ? 1 : ceil_div(q.rows, 4));
             return true;
         case VXB_VARIANT_TCGEN05: case VXB_VARIANT_TCGEN05_WIDE: case VXB_VARIANT_GROUPED_TCGEN05: {
+            if (id == VXB_VARIANT_GROUPED_TCGEN05) {
+                const GroupedFewShape few = grouped_few_shape(q.rows, q.n, (int)sms);   // few rows: weights as the M operand
+                if (few.slots) {
+                    p->tile_rows = few.slots; p->tile_columns = few.channels; p->tile_k = 256;
+                    p->threads = few.threads; p->grid = few.grid;
+                    return true;
+                }
+            }
             const uint32_t tiles = ceil_div(q.rows, v.tile_rows) * ceil_div(q.n, v.tile_columns);
             p->grid = tiles < sms ? tiles : sms;
             return true;

@@ -150,6 +150,13 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
 __device__ __forceinline__ void tmem_ld_wait() {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
+// ... and nothing is computed from these registers before it: the loads only hand their results over here.
+template <uint32_t N>
+__device__ __forceinline__ void tmem_ld_wait(uint32_t (&r)[N]) {
+    tmem_ld_wait();
+#pragma unroll
+    for (uint32_t i = 0; i < N; i++) asm volatile("" : "+r"(r[i]));
+}
 
 // Shared-memory matrix descriptor for a K-major tile whose rows are 128 bytes,
 // 128B-swizzled (what TMA writes with CU_TENSOR_MAP_SWIZZLE_128B): 8-row groups
