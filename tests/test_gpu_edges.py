@@ -82,6 +82,21 @@ def test_word_outputs_on_any_boundary(torch, ctx, n, lead):
     weight.close()
 
 
+@pytest.mark.parametrize("rows,k,n", [(129, 1600, 128), (257, 2048, 100), (512, 2000, 4096), (600, 4096, 1000), (300, 1537, 386)])
+def test_narrow_pair_tiles(torch, ctx, rows, k, n):
+    """Long K and few tiles: 256 x 128 tiles by pairs of CTAs, every kind of output, equal to the single-CTA kernel."""
+    from volvoxai_b200 import w8a8
+    c = wl.single_linear(rows=rows, k=k, n=n, seed=rows + k + n)
+    weight = w8a8.Weight.from_i8(ctx, c["w"], c["ws"], bias_f32=c["bias"], bias_i32=np.arange(n, dtype=np.int32) * 11 - 300)
+    x = dev(torch, c["x"])
+    for call in (lambda r: ctx.linear_acc_i32(weight, x, route=r), lambda r: ctx.linear_f32(weight, x, route=r),
+                 lambda r: ctx.linear_i8(weight, x, 0.1, -5, route=r)):
+        y = call(w8a8.ROUTE_AUTO)
+        assert "pair-narrow" in w8a8.last_route()
+        assert torch.equal(y, call(w8a8.ROUTE_TCGEN05))
+    weight.close()
+
+
 @pytest.mark.parametrize("in_u8", [False, True])
 @pytest.mark.parametrize("rows,k,n", [(1, 128, 40), (40, 48, 33), (128, 256, 130), (130, 16, 65), (200, 1283, 50), (300, 576, 1536),
                                       (700, 2064, 300)])

@@ -182,7 +182,8 @@ struct VxbWeight {
     int32_t* bias_i32 = nullptr;
     int32_t* wsum = nullptr;   // [d_out] sum of codes per channel
     CUtensorMap tmap_b;        // box 256 rows (large-M kernel)
-    CUtensorMap tmap_w128;     // box 128 rows (stream-K decode kernel)
+    CUtensorMap tmap_w128;     // box 128 rows (stream-K decode kernel, pairs of CTAs)
+    CUtensorMap tmap_w64;      // box 64 rows (pairs of CTAs on narrow tiles)
     CUtensorMap tmap_rows;     // box tile_rows rows (channel-owning decode kernel)
     uint32_t tile_rows = 0, tiles_per_cta = 0;
     bool has_tmap = false;
@@ -258,7 +259,8 @@ int finish_weight(VxbContext* ctx, VxbWeight* w, const uint8_t* staging, uint32_
         w->bytes += 4ull * n;
     }
     w->has_tmap = encode_i8_rows(&w->tmap_b, w->w, n, w->kpad, 256) &&
-                  encode_i8_rows(&w->tmap_w128, w->w, n, w->kpad, 128);
+                  encode_i8_rows(&w->tmap_w128, w->w, n, w->kpad, 128) &&
+                  encode_i8_rows(&w->tmap_w64, w->w, n, w->kpad, 64);
     decode_rows_plan(n, ctx->sm_count, &w->tile_rows, &w->tiles_per_cta);
     w->has_tmap = w->has_tmap && encode_i8_rows(&w->tmap_rows, w->w, n, w->kpad, w->tile_rows);
     CUDA_TRY(cudaStreamSynchronize(ctx->stream), -1);
@@ -365,6 +367,7 @@ int run_gemm(VxbContext* ctx, const VxbWeight* w, const int8_t* q, uint32_t rows
     const VxbVariant* variant = vxb_variant_info((uint32_t)plan.variant);
     const bool tensor_map_route = plan.variant == VXB_VARIANT_DECODE_ROWS || plan.variant == VXB_VARIANT_DECODE_STREAMK ||
                                   plan.variant == VXB_VARIANT_TCGEN05 || plan.variant == VXB_VARIANT_TCGEN05_PAIR ||
+                                  plan.variant == VXB_VARIANT_TCGEN05_PAIR_NARROW ||
                                   plan.variant == VXB_VARIANT_GROUPED_TCGEN05;
     if (tensor_map_route && !w->has_tmap) return fail(0, "no tensor map for this weight (driver entry point missing)");
     EpilogueParams ge = epi;
@@ -442,7 +445,7 @@ int run_gemm(VxbContext* ctx, const VxbWeight* w, const int8_t* q, uint32_t rows
             LAUNCH_TRY(launch_decode_tcgen05(a, ctx->sm_count, ctx->stream));
             break;
         }
-        case VXB_VARIANT_TCGEN05: case VXB_VARIANT_TCGEN05_PAIR: case VXB_VARIANT_TCGEN05_WIDE: {
+        case VXB_VARIANT_TCGEN05: case VXB_VARIANT_TCGEN05_PAIR: case VXB_VARIANT_TCGEN05_PAIR_NARROW: case VXB_VARIANT_TCGEN05_WIDE: {
             GemmTcgen05Args a;
             if (!encode_i8_rows(&a.tmap_a, q, rows, q_width ? q_width : w->kpad, 128)) return fail(0, "cuTensorMapEncodeTiled failed for activations");
             a.rows = rows; a.n = w->d_out; a.kpad = w->kpad; a.epi = epi; a.status = ctx->status; a.trace = ctx->trace; a.tma_out = 0;
@@ -457,6 +460,10 @@ int run_gemm(VxbContext* ctx, const VxbWeight* w, const int8_t* q, uint32_t rows
                     a.gather_tma = 1;
                 }
                 LAUNCH_TRY(launch_gemm_pair(a, ctx->stream));
+            } else if (plan.variant == VXB_VARIANT_TCGEN05_PAIR_NARROW) {
+                a.tmap_b = w->tmap_w64;
+                a.gather_tma = 0;
+                LAUNCH_TRY(launch_gemm_pair(a, ctx->stream, true));
             } else if (plan.variant == VXB_VARIANT_TCGEN05_WIDE) {
                 a.tmap_b = w->tmap_b;
                 if (!encode_out32(&a.tmap_out, epi.out, rows, w->d_out, epi.ld)) return fail(0, "cuTensorMapEncodeTiled failed for the output");
@@ -1152,7 +1159,7 @@ int vxb_qlinear_device(VxbContext* ctx, const VxbWeight* w, const void* input, u
         VxbLaunchPlan plan;
         char why[160];
         in_place = vxb_plan(&query, &plan, why, sizeof why) == 1 &&
-                   (plan.variant == VXB_VARIANT_TCGEN05 || plan.variant == VXB_VARIANT_TCGEN05_PAIR);
+                   (plan.variant == VXB_VARIANT_TCGEN05 || plan.variant == VXB_VARIANT_TCGEN05_PAIR || plan.variant == VXB_VARIANT_TCGEN05_PAIR_NARROW);
     }
     if (in_place) return run_gemm(ctx, w, (const int8_t*)input, rows, epi, route, "static+", w->d_in);
     CUDA_TRY(ctx->q.reserve((size_t)rows * w->kpad), 0);

@@ -357,9 +357,10 @@ cudaError_t gemm_tcgen05_prepare();  // one-time func attribute set-up
 // args.tmap_out (args.tma_out must be set)
 cudaError_t launch_gemm_wide(const GemmTcgen05Args& args, int sm_count, cudaStream_t stream);
 // The same GEMM by pairs of CTAs (cta_group::2) on 256 x 256 tiles; tmap_b has a box of 128 rows.
+// narrow: on 256 x 128 tiles, tmap_b with a box of 64 rows; no peers.
 cudaError_t gemm_pair_prepare();    // func attribute + how many pairs can be resident
 int gemm_pair_clusters();           // 0: pairs cannot run on this device
-cudaError_t launch_gemm_pair(const GemmTcgen05Args& args, cudaStream_t stream);
+cudaError_t launch_gemm_pair(const GemmTcgen05Args& args, cudaStream_t stream, bool narrow = false);
 
 // K2g: the GEMM for weights with grouped scales on the tensor cores (fp32 output).  tmap_a and
 // tmap_b have boxes of 128 rows; gscales_t is the group-scale table transposed to

@@ -21,6 +21,11 @@
 //               per warp on the leader's accumulator-empty barrier
 // Two 256-column accumulators per CTA: the epilogue of tile i overlaps the MMAs of tile i+1.
 //
+// The same kernel with 128 channels per tile (64 weight rows per CTA, two 128-column accumulators, four
+// stages) serves launches of few tiles and long K: 24 KB per SM and 128 bytes of K, and twice as many
+// tiles to deal out.  512 x 4096 -> 4096: 64 tiles for 74 pairs, 13.3 us, where 64 tiles of 128 x 256 leave
+// 84 of 148 SMs idle and take 16.8 (the rule: plan.cu).
+//
 // Every copy lands in the shared memory of the CTA that issued it (plain tile loads, one
 // destination each). All mbarrier waits are bounded; a CTA that gives up raises
 // the status word and tells its partner, and both drain, free their TMEM and return.
@@ -34,35 +39,37 @@ namespace {
 using namespace tc;
 
 constexpr uint32_t kBM = 128;           // activation rows per CTA (256 per pair)
-constexpr uint32_t kBNHalf = 128;       // weight rows loaded per CTA
-constexpr uint32_t kBN = 256;           // output channels per tile
 constexpr uint32_t kAtomK = 128;        // K bytes of one swizzle span (one TMA box, four MMAs)
 constexpr uint32_t kAtoms = 2;
 constexpr uint32_t kBK = kAtoms * kAtomK;           // K bytes per stage: two spans, so that the issuing thread's
                                         // per-stage work (barrier wait, commits) is paid once per 8 MMAs
-constexpr uint32_t kStages = 3;
 constexpr uint32_t kAAtomBytes = kBM * kAtomK;     // 16 KiB
-constexpr uint32_t kBAtomBytes = kBNHalf * kAtomK; // 16 KiB
 constexpr uint32_t kABytes = kAtoms * kAAtomBytes;
-constexpr uint32_t kBBytes = kAtoms * kBAtomBytes;
-constexpr uint32_t kStageBytes = kABytes + kBBytes;
-constexpr uint32_t kAccCols = kBN;
-constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kEpiWarps = 8;
 constexpr uint32_t kThreads = 64 + 32 * kEpiWarps + 32;
 constexpr uint32_t kBWarp = 2 + kEpiWarps;
-constexpr uint32_t kEpiCols = kBN / 2;              // columns per epilogue warp
-
-constexpr uint32_t kOffStages = 0;
-constexpr uint32_t kOffWs = kStages * kStageBytes;                   // float[8 warps][128]
-constexpr uint32_t kOffBias = kOffWs + kEpiWarps * kEpiCols * 4;
-constexpr uint32_t kOffStore = kOffBias + kEpiWarps * kEpiCols * 4;   // [8 warps][16 rows x 128 B] store staging
 constexpr uint32_t kStoreBytes = 16 * 128;
-constexpr uint32_t kOffBars = kOffStore + kEpiWarps * kStoreBytes;
-constexpr uint32_t kNumBars = 2 * kStages + 4;
-constexpr uint32_t kOffTmemPtr = kOffBars + kNumBars * 8;
-constexpr uint32_t kOffAbort = kOffTmemPtr + 4;
-constexpr uint32_t kSmemBytes = kOffAbort + 8 + 1024;
+
+// BN output channels per tile: 256, or 128 for launches that cannot fill the chip with tiles of 256
+template <uint32_t BN> struct PairCfg {
+    static constexpr uint32_t kBNHalf = BN / 2;         // weight rows loaded per CTA
+    static constexpr uint32_t kBAtomBytes = kBNHalf * kAtomK;   // 16 / 8 KiB
+    static constexpr uint32_t kBBytes = kAtoms * kBAtomBytes;
+    static constexpr uint32_t kStageBytes = kABytes + kBBytes;
+    static constexpr uint32_t kStages = BN == 256 ? 3 : 4;
+    static constexpr uint32_t kTmemCols = 2 * BN;       // two accumulators
+    static constexpr uint32_t kEpiCols = BN / 2;        // columns per epilogue warp
+    static constexpr uint32_t kOffStages = 0;
+    static constexpr uint32_t kOffWs = kStages * kStageBytes;                   // float[8 warps][kEpiCols]
+    static constexpr uint32_t kOffBias = kOffWs + kEpiWarps * kEpiCols * 4;
+    static constexpr uint32_t kOffStore = kOffBias + kEpiWarps * kEpiCols * 4;   // [8 warps] store tiles
+    static constexpr uint32_t kOffBars = kOffStore + kEpiWarps * kStoreBytes;
+    static constexpr uint32_t kNumBars = 2 * kStages + 4;
+    static constexpr uint32_t kOffTmemPtr = kOffBars + kNumBars * 8;
+    static constexpr uint32_t kOffAbort = kOffTmemPtr + 4;
+    static constexpr uint32_t kSmemBytes = kOffAbort + 8 + 1024;
+    static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
+};
 
 // ---- cluster-scope PTX ----------------------------------------------------------------------
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -139,23 +146,27 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar_cluster) {
                  ::"r"(bar_cluster) : "memory");
 }
 
-struct Smem {
+template <uint32_t BN> struct Smem {
+    using C = PairCfg<BN>;
     uint8_t* base;
-    __device__ uint32_t a(uint32_t s) const { return smem_u32(base + kOffStages + s * kStageBytes); }
+    __device__ uint32_t a(uint32_t s) const { return smem_u32(base + C::kOffStages + s * C::kStageBytes); }
     __device__ uint32_t b(uint32_t s) const { return a(s) + kABytes; }
-    __device__ uint32_t full(uint32_t s) const { return smem_u32(base + kOffBars + s * 8); }
-    __device__ uint32_t empty(uint32_t s) const { return smem_u32(base + kOffBars + (kStages + s) * 8); }
-    __device__ uint32_t tmem_full(uint32_t b) const { return smem_u32(base + kOffBars + (2 * kStages + b) * 8); }
-    __device__ uint32_t tmem_empty(uint32_t b) const { return smem_u32(base + kOffBars + (2 * kStages + 2 + b) * 8); }
-    __device__ uint32_t* tmem_ptr() const { return reinterpret_cast<uint32_t*>(base + kOffTmemPtr); }
-    __device__ volatile int* abort_flag() const { return reinterpret_cast<volatile int*>(base + kOffAbort); }
-    __device__ float* ws() const { return reinterpret_cast<float*>(base + kOffWs); }
-    __device__ float* bias() const { return reinterpret_cast<float*>(base + kOffBias); }
+    __device__ uint32_t full(uint32_t s) const { return smem_u32(base + C::kOffBars + s * 8); }
+    __device__ uint32_t empty(uint32_t s) const { return smem_u32(base + C::kOffBars + (C::kStages + s) * 8); }
+    __device__ uint32_t tmem_full(uint32_t b) const { return smem_u32(base + C::kOffBars + (2 * C::kStages + b) * 8); }
+    __device__ uint32_t tmem_empty(uint32_t b) const { return smem_u32(base + C::kOffBars + (2 * C::kStages + 2 + b) * 8); }
+    __device__ uint32_t* tmem_ptr() const { return reinterpret_cast<uint32_t*>(base + C::kOffTmemPtr); }
+    __device__ volatile int* abort_flag() const { return reinterpret_cast<volatile int*>(base + C::kOffAbort); }
+    __device__ float* ws() const { return reinterpret_cast<float*>(base + C::kOffWs); }
+    __device__ float* bias() const { return reinterpret_cast<float*>(base + C::kOffBias); }
 };
 
+template <uint32_t BN>
 __device__ __forceinline__ void gemm_i8_pair_body(const GemmTcgen05Args& args) {
     extern __shared__ uint8_t smem_raw[];
-    Smem sm;
+    using C = PairCfg<BN>;
+    constexpr uint32_t kBN = BN, kAccCols = BN;
+    Smem<BN> sm;
     sm.base = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();            // 0 = leader (issues the pair's MMAs)
@@ -168,7 +179,7 @@ __device__ __forceinline__ void gemm_i8_pair_body(const GemmTcgen05Args& args) {
     volatile int* abort_flag = sm.abort_flag();
 
     if (threadIdx.x == 0) {
-        for (uint32_t s = 0; s < kStages; s++) { mbar_init(sm.full(s), 1); mbar_init(sm.empty(s), 1); }
+        for (uint32_t s = 0; s < C::kStages; s++) { mbar_init(sm.full(s), 1); mbar_init(sm.empty(s), 1); }
         // accumulator-empty: one arrival per epilogue warp of both CTAs (only the leader's is waited on)
         for (uint32_t b = 0; b < 2; b++) { mbar_init(sm.tmem_full(b), 1); mbar_init(sm.tmem_empty(b), 2 * kEpiWarps); }
         arm_abort(abort_flag, args.status);
@@ -178,7 +189,7 @@ __device__ __forceinline__ void gemm_i8_pair_body(const GemmTcgen05Args& args) {
         pdl_release();   // the next launch in the stream may begin its own prologue
     }
     if (warp == 1) {
-        tmem_alloc_pair(smem_u32(sm.tmem_ptr()), kTmemCols);
+        tmem_alloc_pair(smem_u32(sm.tmem_ptr()), C::kTmemCols);
         tmem_relinquish_pair();
     }
     tc_fence_before();
@@ -198,11 +209,11 @@ __device__ __forceinline__ void gemm_i8_pair_body(const GemmTcgen05Args& args) {
                 for (uint32_t kb = 0; kb < num_kb; kb++) {
                     if (!mbar_wait(sm.empty(stage), phase ^ 1u, abort_flag)) { ok = false; break; }
                     // the leader's barrier collects the bytes of both CTAs' copies of the stage
-                    if (rank == 0) mbar_expect_tx(sm.full(stage), 2 * kStageBytes);
+                    if (rank == 0) mbar_expect_tx(sm.full(stage), 2 * C::kStageBytes);
 #pragma unroll
                     for (uint32_t a = 0; a < kAtoms; a++)
                         tma_load_2d_pair(sm.a(stage) + a * kAAtomBytes, &args.tmap_a, in_cta(sm.full(stage), 0), (int32_t)(kb * kBK + a * kAtomK), m0);
-                    if (++stage == kStages) { stage = 0; phase ^= 1u; }
+                    if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
                 }
             }
         }
@@ -212,13 +223,13 @@ __device__ __forceinline__ void gemm_i8_pair_body(const GemmTcgen05Args& args) {
             uint32_t stage = 0, phase = 0;
             bool ok = true;
             for (uint32_t t = pair; ok && t < total_tiles; t += pairs) {
-                const int32_t n0 = (int32_t)((t / tiles_m) * kBN + rank * kBNHalf);
+                const int32_t n0 = (int32_t)((t / tiles_m) * kBN + rank * C::kBNHalf);
                 for (uint32_t kb = 0; kb < num_kb; kb++) {
                     if (!mbar_wait(sm.empty(stage), phase ^ 1u, abort_flag)) { ok = false; break; }
 #pragma unroll
                     for (uint32_t a = 0; a < kAtoms; a++)
-                        tma_load_2d_pair(sm.b(stage) + a * kBAtomBytes, &args.tmap_b, in_cta(sm.full(stage), 0), (int32_t)(kb * kBK + a * kAtomK), n0);
-                    if (++stage == kStages) { stage = 0; phase ^= 1u; }
+                        tma_load_2d_pair(sm.b(stage) + a * C::kBAtomBytes, &args.tmap_b, in_cta(sm.full(stage), 0), (int32_t)(kb * kBK + a * kAtomK), n0);
+                    if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
                 }
             }
         }
@@ -245,7 +256,7 @@ __device__ __forceinline__ void gemm_i8_pair_body(const GemmTcgen05Args& args) {
                     umma_i8_pair_lo(d_tmem, a_lo + 6u, b_lo + 6u, idesc);
 #pragma unroll
                     for (uint32_t a = 1; a < kAtoms; a++) {   // the other spans' tiles
-                        const uint32_t a2 = a_lo + a * (kAAtomBytes >> 4), b2 = b_lo + a * (kBAtomBytes >> 4);
+                        const uint32_t a2 = a_lo + a * (kAAtomBytes >> 4), b2 = b_lo + a * (C::kBAtomBytes >> 4);
                         umma_i8_pair_lo(d_tmem, a2, b2, idesc);
                         umma_i8_pair_lo(d_tmem, a2 + 2u, b2 + 2u, idesc);
                         umma_i8_pair_lo(d_tmem, a2 + 4u, b2 + 4u, idesc);
@@ -254,8 +265,8 @@ __device__ __forceinline__ void gemm_i8_pair_body(const GemmTcgen05Args& args) {
                     // the stage is free again in both CTAs once these MMAs have read it
                     umma_commit_pair(empty_s);
                     umma_commit_pair(empty_s + peer_delta);
-                    full_s += 8; empty_s += 8; a_lo += kStageBytes >> 4;
-                    if (++stage == kStages) { stage = 0; phase ^= 1u; full_s = sm.full(0); empty_s = sm.empty(0); a_lo = a_lo0; }
+                    full_s += 8; empty_s += 8; a_lo += C::kStageBytes >> 4;
+                    if (++stage == C::kStages) { stage = 0; phase ^= 1u; full_s = sm.full(0); empty_s = sm.empty(0); a_lo = a_lo0; }
                 }
                 if (!ok) break;
                 umma_commit_pair(sm.tmem_full(acc));
@@ -268,10 +279,10 @@ __device__ __forceinline__ void gemm_i8_pair_body(const GemmTcgen05Args& args) {
         // ---------------- epilogue (warps 2..9): this CTA's 128 rows x 256 columns ----------------
         const uint32_t quarter = warp & 3u;              // TMEM lanes [32*quarter, +32)
         const uint32_t half = (warp - 2u) >> 2;          // columns [128*half, +128) of the tile
-        const uint32_t cbase = half * kEpiCols;
+        const uint32_t cbase = half * C::kEpiCols;
         const EpilogueParams& ep = args.epi;
-        float* s_ws = sm.ws() + (warp - 2u) * kEpiCols;
-        float* s_bias = sm.bias() + (warp - 2u) * kEpiCols;
+        float* s_ws = sm.ws() + (warp - 2u) * C::kEpiCols;
+        float* s_bias = sm.bias() + (warp - 2u) * C::kEpiCols;
         const float zero_f = __int2float_rn(ep.out_zero);
         const float lo_f = __int2float_rn(ep.out_lo), hi_f = __int2float_rn(ep.out_hi);
         // every 32-column chunk of a row starts on 16 bytes (a chunk of the SiLU * Mul tail is 16 outputs wide)
@@ -282,12 +293,12 @@ __device__ __forceinline__ void gemm_i8_pair_body(const GemmTcgen05Args& args) {
         // fused all-gather (int8 output, aligned buffers): 64 columns at a time leave through this warp's
         // 2 KB staging tile ([32 rows x 64 B], 64B-swizzled) as one TMA tile store per destination
         const bool gather = ep.n_peers != 0;
-        const uint32_t gbuf = smem_u32(sm.base + kOffStore + (warp - 2u) * kStoreBytes);
+        const uint32_t gbuf = smem_u32(sm.base + C::kOffStore + (warp - 2u) * kStoreBytes);
         pdl_wait();   // row scales and residual come from earlier launches, and one may still read the output
         for (uint32_t t = pair; ok && t < total_tiles; t += pairs) {
             const uint32_t m0 = (t % tiles_m) * 2 * kBM + rank * kBM, n0 = (t / tiles_m) * kBN + cbase;
             __syncwarp();
-            for (uint32_t i = lane; i < kEpiCols; i += 32) {
+            for (uint32_t i = lane; i < C::kEpiCols; i += 32) {
                 const uint32_t n = n0 + i;
                 float wsv = 0.0f, bv = 0.0f;
                 if (n < args.n && ep.mode != kEpiAcc) {
@@ -308,7 +319,7 @@ __device__ __forceinline__ void gemm_i8_pair_body(const GemmTcgen05Args& args) {
             const bool fast = ep.fast_div != 0 && div_const_row_ok(as);
             const uint32_t taddr = tmem_base + ((quarter * 32u) << 16) + acc * kAccCols + cbase;
 #pragma unroll 1
-            for (uint32_t c = 0; c < kEpiCols; c += 32) {
+            for (uint32_t c = 0; c < C::kEpiCols; c += 32) {
                 uint32_t r[32];
                 tmem_ld32(taddr + c, r);
                 tmem_ld_wait();
@@ -326,7 +337,7 @@ __device__ __forceinline__ void gemm_i8_pair_body(const GemmTcgen05Args& args) {
                 const bool full = col + 32 <= args.n;
                 // this warp's store tile, its first row and how many of its 32 rows exist (made where they are used:
                 // held throughout the loop they cost registers that the epilogue needs)
-                auto store_tile = [&] { return sm.base + kOffStore + (warp - 2u) * kStoreBytes; };
+                auto store_tile = [&] { return sm.base + C::kOffStore + (warp - 2u) * kStoreBytes; };
                 auto first_row = [&] { return m0 + quarter * 32u; };
                 auto live_rows = [&] { const uint32_t r0 = first_row(); return r0 >= args.rows ? 0u : args.rows - r0 < 32u ? args.rows - r0 : 32u; };
                 const float4* w4 = reinterpret_cast<const float4*>(s_ws + c);
@@ -493,48 +504,60 @@ __device__ __forceinline__ void gemm_i8_pair_body(const GemmTcgen05Args& args) {
     // still target it
     cluster_sync_all();
     tc_fence_after();
-    if (warp == 1) tmem_dealloc_pair(tmem_base, kTmemCols);
+    if (warp == 1) tmem_dealloc_pair(tmem_base, C::kTmemCols);
 }
 
+template <uint32_t BN>
 __global__ void __launch_bounds__(kThreads, 1)
-gemm_i8_pair_kernel(const __grid_constant__ GemmTcgen05Args args) { gemm_i8_pair_body(args); }
+gemm_i8_pair_kernel(const __grid_constant__ GemmTcgen05Args args) { gemm_i8_pair_body<BN>(args); }
 
 int g_pair_clusters = 0;   // co-resident clusters of two, queried once
 
-}  // namespace
-
-cudaError_t gemm_pair_prepare() {
-    cudaError_t e = cudaFuncSetAttribute(gemm_i8_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
+template <uint32_t BN>
+cudaError_t prepare(int* clusters) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_i8_pair_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PairCfg<BN>::kSmemBytes);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2); cfg.blockDim = dim3(kThreads); cfg.dynamicSmemBytes = kSmemBytes;
+    cfg.gridDim = dim3(2); cfg.blockDim = dim3(kThreads); cfg.dynamicSmemBytes = PairCfg<BN>::kSmemBytes;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr; cfg.numAttrs = 1;
-    int clusters = 0;
-    e = cudaOccupancyMaxActiveClusters(&clusters, gemm_i8_pair_kernel, &cfg);
-    if (e != cudaSuccess) return e;
-    g_pair_clusters = clusters;
-    return cudaSuccess;
+    return cudaOccupancyMaxActiveClusters(clusters, gemm_i8_pair_kernel<BN>, &cfg);
 }
 
-int gemm_pair_clusters() { return g_pair_clusters; }
-
-cudaError_t launch_gemm_pair(const GemmTcgen05Args& args, cudaStream_t stream) {
-    if (args.rows == 0 || args.n == 0) return cudaSuccess;
-    if (g_pair_clusters <= 0 || (args.epi.n_peers != 0 && (!args.gather_tma || args.epi.mode != kEpiI8))) return cudaErrorInvalidValue;
-    const uint32_t tiles = ((args.rows + 2 * kBM - 1) / (2 * kBM)) * ((args.n + kBN - 1) / kBN);
+template <uint32_t BN>
+cudaError_t launch_pair(const GemmTcgen05Args& args, cudaStream_t stream) {
+    const uint32_t tiles = ((args.rows + 2 * kBM - 1) / (2 * kBM)) * ((args.n + BN - 1) / BN);
     const uint32_t pairs = tiles < (uint32_t)g_pair_clusters ? tiles : (uint32_t)g_pair_clusters;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * pairs); cfg.blockDim = dim3(kThreads); cfg.dynamicSmemBytes = kSmemBytes; cfg.stream = stream;
+    cfg.gridDim = dim3(2 * pairs); cfg.blockDim = dim3(kThreads); cfg.dynamicSmemBytes = PairCfg<BN>::kSmemBytes; cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // set-up and weight loads under the predecessor's tail
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr; cfg.numAttrs = 2;
-    return cudaLaunchKernelEx(&cfg, gemm_i8_pair_kernel, args);
+    return cudaLaunchKernelEx(&cfg, gemm_i8_pair_kernel<BN>, args);
+}
+
+}  // namespace
+
+cudaError_t gemm_pair_prepare() {
+    int wide = 0, narrow = 0;
+    cudaError_t e = prepare<256>(&wide);
+    if (e == cudaSuccess) e = prepare<128>(&narrow);
+    if (e != cudaSuccess) return e;
+    g_pair_clusters = wide < narrow ? wide : narrow;
+    return cudaSuccess;
+}
+
+int gemm_pair_clusters() { return g_pair_clusters; }
+
+cudaError_t launch_gemm_pair(const GemmTcgen05Args& args, cudaStream_t stream, bool narrow) {
+    if (args.rows == 0 || args.n == 0) return cudaSuccess;
+    if (g_pair_clusters <= 0 || (args.epi.n_peers != 0 && (narrow || !args.gather_tma || args.epi.mode != kEpiI8))) return cudaErrorInvalidValue;
+    return narrow ? launch_pair<128>(args, stream) : launch_pair<256>(args, stream);
 }
 
 }  // namespace vxb

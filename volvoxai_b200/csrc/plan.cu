@@ -115,7 +115,7 @@ bool geometry(VxbVariantId id, const VxbPlanQuery& q, VxbLaunchPlan* p) {
             p->grid = tiles < sms ? tiles : sms;
             return true;
         }
-        case VXB_VARIANT_TCGEN05_PAIR: {
+        case VXB_VARIANT_TCGEN05_PAIR: case VXB_VARIANT_TCGEN05_PAIR_NARROW: {
             const uint32_t tiles = ceil_div(q.rows, v.tile_rows) * ceil_div(q.n, v.tile_columns);
             p->grid = 2 * (tiles < q.pair_clusters ? tiles : q.pair_clusters);
             return true;
@@ -218,6 +218,20 @@ int vxb_plan(const VxbPlanQuery* query, VxbLaunchPlan* out, char* why, uint32_t 
             // pairs of CTAs on 256 x 256 tiles once there are at least two waves of 128 x 256 tiles
             const uint32_t tiles = ceil_div(q.rows, 128) * ceil_div(q.n, 256);
             chosen = (q.pair_clusters > 0 && tiles >= 2u * sms) ? VXB_VARIANT_TCGEN05_PAIR : VXB_VARIANT_TCGEN05;
+            if (q.pair_clusters > 0 && round_up(q.k, kKAlign) > VXB_WIDE_MAX_KPAD) {
+                // Long K: a wave of tiles costs its K loop, bound by the operands an SM pulls from L2 per 128 bytes of
+                // K (48 KB for 128 x 256 alone, 32 KB in a pair on 256 x 256, 24 KB on 256 x 128) or by the MMAs on
+                // them (512, 512, 256 clocks); a pair takes longer to set up.  In clocks, from K = 4096 -> 4096 with
+                // fp32 output: 512 rows 16.8 / 16.7 / 13.3 us, 1024 rows 17.1 / 17.8 / -, 2048 rows 29.3 / 27.4 / -
+                // (alone / pair / narrow pair).
+                const uint32_t pair_rows = ceil_div(q.rows, 256);
+                const uint64_t kb = round_up(q.k, kKAlign) / kKAlign;
+                const uint64_t alone = 9300ull + 724ull * kb * ceil_div(tiles, sms);
+                const uint64_t pair = 14250ull + 594ull * kb * ceil_div(pair_rows * ceil_div(q.n, 256), q.pair_clusters);
+                const uint64_t narrow = 13000ull + 386ull * kb * ceil_div(pair_rows * ceil_div(q.n, 128), q.pair_clusters);
+                chosen = narrow < pair && narrow < alone ? VXB_VARIANT_TCGEN05_PAIR_NARROW
+                       : pair <= alone ? VXB_VARIANT_TCGEN05_PAIR : VXB_VARIANT_TCGEN05;
+            }
             // 32-bit outputs at short K are bound by the output, not by the tensor pipe
             char unused[8];
             if (q.epilogue != VXB_EPI_I8 && round_up(q.k, kKAlign) <= VXB_WIDE_MAX_KPAD &&
