@@ -48,6 +48,7 @@ extern "C" {
 #define VXB_VF_FUSED_K1 16u   /* quantizes the fp32 rows itself: one launch per linear, fp32 input only */
 #define VXB_VF_TILE_STORE 32u /* 32-bit outputs leave as TMA tile stores: output base, row pitch and width multiples of 16 bytes, \
                                  residual Add as the only fused tail */
+#define VXB_VF_SILU_STORE 64u /* the SiLU*Mul tail and nothing else, fp32, leaving as TMA tile stores (same alignment) */
 
 /*
  * Variant rows.  Fields:
@@ -67,6 +68,7 @@ extern "C" {
     X(TCGEN05_PAIR,     6, "tcgen05-pair-i8",           "gemm_i8_pair_kernel",          256, 256, 256, 352, 2, 223000,   1,   0, 7u, 1u, 0, 1u | 2u | 4u,  650) \
     X(TCGEN05_PAIR_NARROW, 0, "tcgen05-pair-narrow-i8", "gemm_i8_pair_kernel",          256, 128, 256, 352, 2, 223000,   1,   0, 7u, 1u, 0, 1u | 4u,       645) \
     X(TCGEN05_WIDE,     8, "tcgen05-wide-i8",           "gemm_i8_wide_kernel",          128, 256, 128, 608, 1, 231000,   1,   0, 3u, 1u, 0, 1u | 4u | 32u, 640) \
+    X(TCGEN05_WIDE_SILU, 0, "tcgen05-wide-silu-i8",    "gemm_i8_wide_kernel",          128, 256, 128, 608, 1, 231000,   1,   0, 2u, 1u, 0, 1u | 4u | 64u, 641) \
     X(GROUPED_TCGEN05,  0, "tcgen05-grouped-i8",        "gemm_i8_grouped_tcgen05_kernel", 128, 128, 128, 320, 1, 223000,   1,   0, 2u, 6u, 0, 1u,           500) \
     X(GEMV_GROUPED,     0, "gemv-grouped",              "gemv_grouped_kernel",            0,   0,   0, 256, 1,  65536,   1,   4, 2u, 6u, 0, 1u,           550) \
     X(GEMV_W4_GROUPED,  0, "gemv-w4-grouped",           "gemv_w4_grouped_kernel",         0,   0,   0, 256, 1,  65536,   1,   2, 2u, 4u, 0, 1u,           560) \

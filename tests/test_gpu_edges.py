@@ -171,6 +171,25 @@ def test_grouped_few_rows(torch, ctx, oracle, group, rows, k, n):
     wg.close()
 
 
+@pytest.mark.parametrize("rows,k,n", [(1200, 100, 4096), (2500, 576, 2064), (4097, 65, 1304)])
+def test_wide_silu_tiles(torch, ctx, rows, k, n):
+    """A full wave of tiles: the SiLU * Mul tail through TMA tile stores, ragged rows, a last tile half empty, a row pitch
+    wider than the output; bit-equal to the general kernel's tail (the same operations), which an unaligned output takes."""
+    from volvoxai_b200 import w8a8
+    c = wl.single_linear(rows=rows, k=k, n=n, seed=rows + n)
+    weight = w8a8.Weight.from_i8(ctx, c["w"], c["ws"], bias_f32=c["bias"])
+    x = dev(torch, c["x"])
+    wide = torch.full((rows, n // 2 + 8), 99.0, device="cuda")
+    ctx.linear_f32_fused(weight, x, silu_mul=True, out=wide[:, 4:4 + n // 2])
+    assert "wide-silu" in w8a8.last_route()
+    odd = torch.full((rows, n // 2 + 1), 99.0, device="cuda")
+    ctx.linear_f32_fused(weight, x, silu_mul=True, out=odd[:, 1:])
+    assert "wide" not in w8a8.last_route()
+    assert torch.equal(wide[:, 4:4 + n // 2], odd[:, 1:])
+    assert (wide[:, :4] == 99).all() and (wide[:, 4 + n // 2:] == 99).all()
+    weight.close()
+
+
 @pytest.mark.parametrize("rows,k", [(1, 64), (5, 1000), (64, 1024), (700, 576), (40, 9000)])
 def test_rmsnorm_products_near_and_far_from_one(torch, ctx, rows, k):
     """The normalized rows against the same arithmetic in 64 bits: ordinary rows, rows scaled to 1e-25 and 1e25 (the

@@ -312,7 +312,8 @@ VxbPlanQuery plan_query(const VxbContext* ctx, const VxbWeight* w, uint32_t rows
     query.requested_route = requested; query.n_peers = epi.n_peers;
     query.fused_tail = (epi.residual ? 1u : 0u) | (epi.act ? 2u : 0u);
     // TMA tile stores clip at the matrix edge in units of 16 bytes: the width must be a multiple of four 32-bit columns too
-    query.out_store_aligned = (epi.mode != kEpiI8 && !((uintptr_t)epi.out & 15u) && !(epi.ld & 3u) && !(w->d_out & 3u)) ? 1u : 0u;
+    query.out_store_aligned = (epi.mode != kEpiI8 && !((uintptr_t)epi.out & 15u) && !(epi.ld & 3u) &&
+                               !((epi.act ? w->d_out >> 1 : w->d_out) & 3u)) ? 1u : 0u;
     if (epi.mode == kEpiI8 && epi.n_peers) {
         bool aligned = !((uintptr_t)epi.out & 15u) && !(epi.ld & 15u) && !(w->d_out & 15u) && tunables().gather_tma;
         for (uint32_t p = 0; p < epi.n_peers; p++) aligned = aligned && !((uintptr_t)epi.peer_out[p] & 15u);
@@ -445,7 +446,8 @@ int run_gemm(VxbContext* ctx, const VxbWeight* w, const int8_t* q, uint32_t rows
             LAUNCH_TRY(launch_decode_tcgen05(a, ctx->sm_count, ctx->stream));
             break;
         }
-        case VXB_VARIANT_TCGEN05: case VXB_VARIANT_TCGEN05_PAIR: case VXB_VARIANT_TCGEN05_PAIR_NARROW: case VXB_VARIANT_TCGEN05_WIDE: {
+        case VXB_VARIANT_TCGEN05: case VXB_VARIANT_TCGEN05_PAIR: case VXB_VARIANT_TCGEN05_PAIR_NARROW: case VXB_VARIANT_TCGEN05_WIDE:
+        case VXB_VARIANT_TCGEN05_WIDE_SILU: {
             GemmTcgen05Args a;
             if (!encode_i8_rows(&a.tmap_a, q, rows, q_width ? q_width : w->kpad, 128)) return fail(0, "cuTensorMapEncodeTiled failed for activations");
             a.rows = rows; a.n = w->d_out; a.kpad = w->kpad; a.epi = epi; a.status = ctx->status; a.trace = ctx->trace; a.tma_out = 0;
@@ -464,9 +466,9 @@ int run_gemm(VxbContext* ctx, const VxbWeight* w, const int8_t* q, uint32_t rows
                 a.tmap_b = w->tmap_w64;
                 a.gather_tma = 0;
                 LAUNCH_TRY(launch_gemm_pair(a, ctx->stream, true));
-            } else if (plan.variant == VXB_VARIANT_TCGEN05_WIDE) {
+            } else if (plan.variant == VXB_VARIANT_TCGEN05_WIDE || plan.variant == VXB_VARIANT_TCGEN05_WIDE_SILU) {
                 a.tmap_b = w->tmap_b;
-                if (!encode_out32(&a.tmap_out, epi.out, rows, w->d_out, epi.ld)) return fail(0, "cuTensorMapEncodeTiled failed for the output");
+                if (!encode_out32(&a.tmap_out, epi.out, rows, epi.act ? w->d_out >> 1 : w->d_out, epi.ld)) return fail(0, "cuTensorMapEncodeTiled failed for the output");
                 a.tma_out = 1;
                 LAUNCH_TRY(launch_gemm_wide(a, ctx->sm_count, ctx->stream));
             } else {

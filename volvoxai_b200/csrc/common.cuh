@@ -231,7 +231,7 @@ __device__ __forceinline__ void epi_f32_2(int32_t acc0, int32_t acc1, uint64_t a
 // silu(g) * u as the reference's fused gate/up decode kernel computes it (g * sigmoid(g), then * u;
 // native/src/backends/cuda/kernels/cuda_forward_gemv_pair_kernels.inc:457-459), with an accurate exp.
 __device__ __forceinline__ float epi_silu_mul(float gate, float up) {
-    const float sig = __fdiv_rn(1.0f, __fadd_rn(1.0f, expf(-gate)));
+    const float sig = __frcp_rn(__fadd_rn(1.0f, expf(-gate)));   // the IEEE quotient 1 / x
     return __fmul_rn(__fmul_rn(gate, sig), up);
 }
 
@@ -354,7 +354,7 @@ cudaError_t launch_gemm_tcgen05(const GemmTcgen05Args& args, int sm_count, cudaS
 inline bool gather_is_link_bound(uint32_t n_peers, uint32_t kpad) { return n_peers != 0 && (uint64_t)n_peers * 2140u > kpad; }
 cudaError_t gemm_tcgen05_prepare();  // one-time func attribute set-up
 // K2w: the GEMM for 32-bit outputs (fp32 / raw int32) with sixteen epilogue warps and TMA tile stores through
-// args.tmap_out (args.tma_out must be set)
+// args.tmap_out (args.tma_out must be set); with epi.act the SiLU * Mul form, tmap_out n / 2 wide
 cudaError_t launch_gemm_wide(const GemmTcgen05Args& args, int sm_count, cudaStream_t stream);
 // The same GEMM by pairs of CTAs (cta_group::2) on 256 x 256 tiles; tmap_b has a box of 128 rows.
 // narrow: on 256 x 128 tiles, tmap_b with a box of 64 rows; no peers.

@@ -15,6 +15,9 @@
 //     its 128-byte row into a 128B-swizzled [32 rows x 128 B] staging tile, one lane issues
 //     cp.async.bulk.tensor (shared -> global, clipped by the tensor map at the matrix edges, no
 //     multicast), and the warp goes on with the next chunk while the store drains.
+//   * The SiLU * Mul tail (SILU = true, 32 outputs per warp and tile) has a form of its own: an exponential and a
+//     reciprocal per output are latency that eight warps left exposed as well.  4096 x 576 -> 2 x 1536: a layer
+//     with it 87.6 -> 82.4 us (and 128 with the tail's outputs stored one word per row and instruction).
 //   * Three 48 KB pipeline stages instead of four: the fourth stage's room is the sixteen staging tiles.
 //   * 96 registers per thread (608 threads), which only this epilogue fits in; the requantizing
 //     epilogues stay in the general kernel.
@@ -73,6 +76,7 @@ __device__ __forceinline__ void stamp(unsigned long long* trace, uint32_t slot) 
     }
 }
 
+template <bool SILU>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_i8_wide_kernel(const __grid_constant__ GemmTcgen05Args args) {
     extern __shared__ uint8_t smem_raw[];
@@ -230,7 +234,7 @@ gemm_i8_wide_kernel(const __grid_constant__ GemmTcgen05Args args) {
                         epi_f32_2((int32_t)r[4 * j + 0], (int32_t)r[4 * j + 1], as2, f32x2(wv.x, wv.y), bv.x, bv.y, r[4 * j + 0], r[4 * j + 1]);
                         epi_f32_2((int32_t)r[4 * j + 2], (int32_t)r[4 * j + 3], as2, f32x2(wv.z, wv.w), bv.z, bv.w, r[4 * j + 2], r[4 * j + 3]);
                     }
-                    if (ep.residual && row_ok) {
+                    if (!SILU && ep.residual && row_ok) {
                         // fused residual addition: y += residual[row, col ...]
                         const float* res = ep.residual + (size_t)row * ep.ld_res + col;
                         if (col + 32 <= args.n && (((uintptr_t)res) & 15u) == 0) {
@@ -248,6 +252,32 @@ gemm_i8_wide_kernel(const __grid_constant__ GemmTcgen05Args args) {
                                 if (col + i < args.n) r[i] = __float_as_uint(__fadd_rn(__uint_as_float(r[i]), __ldg(res + i)));
                         }
                     }
+                }
+                if constexpr (SILU) {
+                    // channel pairs (gate, up) -> silu(gate) * up: this warp's two chunks are the left and right half
+                    // of one 32-column tile, which leaves after the second (or last) of them
+                    if (c == 0) {
+                        if (lane == 0) tma_store_wait_read();
+                        __syncwarp();
+                    }
+#pragma unroll
+                    for (uint32_t j = 0; j < 4; j++) {
+                        float y[4];
+#pragma unroll
+                        for (uint32_t i = 0; i < 4; i++) y[i] = epi_silu_mul(__uint_as_float(r[8 * j + 2 * i]), __uint_as_float(r[8 * j + 2 * i + 1]));
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};"
+                                     ::"r"(out_tile + lane * 128u + ((((c >> 3) + j) ^ (lane & 7u)) << 4)),
+                                       "r"(__float_as_uint(y[0])), "r"(__float_as_uint(y[1])), "r"(__float_as_uint(y[2])), "r"(__float_as_uint(y[3])) : "memory");
+                    }
+                    if (c != 0 || col + 32 >= args.n) {
+                        fence_proxy_async();
+                        __syncwarp();
+                        if (lane == 0) {
+                            tma_store_2d(&args.tmap_out, out_tile, (int32_t)(n0 >> 1), (int32_t)(m0 + quarter * 32u));
+                            tma_store_commit();
+                        }
+                    }
+                    continue;
                 }
                 if (lane == 0) tma_store_wait_read();          // the previous chunk's store has left the tile
                 __syncwarp();
@@ -291,16 +321,20 @@ gemm_i8_wide_kernel(const __grid_constant__ GemmTcgen05Args args) {
 
 }  // namespace
 
-cudaError_t gemm_wide_prepare() { return ensure_dynamic_smem<gemm_i8_wide_kernel>(kSmemBytes); }
+cudaError_t gemm_wide_prepare(bool silu) {
+    return silu ? ensure_dynamic_smem<gemm_i8_wide_kernel<true>>(kSmemBytes) : ensure_dynamic_smem<gemm_i8_wide_kernel<false>>(kSmemBytes);
+}
 
 cudaError_t launch_gemm_wide(const GemmTcgen05Args& args, int sm_count, cudaStream_t stream) {
     const uint32_t tiles = ((args.rows + kBM - 1) / kBM) * ((args.n + kBN - 1) / kBN);
     if (!tiles) return cudaSuccess;
     if (args.kpad % kBK != 0 || !args.tma_out) return cudaErrorInvalidValue;
-    cudaError_t e = gemm_wide_prepare();
+    const bool silu = args.epi.act == 1u;
+    if (silu && (args.epi.mode != kEpiF32 || args.epi.residual)) return cudaErrorInvalidValue;
+    cudaError_t e = gemm_wide_prepare(silu);
     if (e != cudaSuccess) return e;
     const uint32_t grid = tiles < (uint32_t)sm_count ? tiles : (uint32_t)sm_count;
-    return launch_pdl(gemm_i8_wide_kernel, dim3(grid), dim3(kThreads), kSmemBytes, stream, args);
+    return launch_pdl(silu ? gemm_i8_wide_kernel<true> : gemm_i8_wide_kernel<false>, dim3(grid), dim3(kThreads), kSmemBytes, stream, args);
 }
 
 }  // namespace vxb

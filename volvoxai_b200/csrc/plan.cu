@@ -51,6 +51,10 @@ bool admitted(const VxbVariant& v, const VxbPlanQuery& q, char* why, uint32_t by
         if (!q.out_store_aligned) { refuse(why, bytes, "%s needs a 16-byte aligned output base and row pitch", v.id); return false; }
         if (q.fused_tail & 2u) { refuse(why, bytes, "%s has no SiLU*Mul tail", v.id); return false; }
     }
+    if ((v.flags & VXB_VF_SILU_STORE) && (!q.out_store_aligned || q.fused_tail != 2u)) {
+        refuse(why, bytes, "%s is the SiLU*Mul tail into a 16-byte aligned output", v.id);
+        return false;
+    }
     if (v.cluster > 1 && q.pair_clusters == 0) { refuse(why, bytes, "no co-resident CTA pairs on this device"); return false; }
     if (v.flags & VXB_VF_FUSED_K1) {
         if (!q.fp32_input) { refuse(why, bytes, "%s starts from fp32 rows", v.id); return false; }
@@ -102,7 +106,7 @@ bool geometry(VxbVariantId id, const VxbPlanQuery& q, VxbLaunchPlan* p) {
         case VXB_VARIANT_DP4A_GROUPED:
             p->grid = ceil_div(q.n, 128) * (q.rows == 1 ? 1 : ceil_div(q.rows, 4));
             return true;
-        case VXB_VARIANT_TCGEN05: case VXB_VARIANT_TCGEN05_WIDE: case VXB_VARIANT_GROUPED_TCGEN05: {
+        case VXB_VARIANT_TCGEN05: case VXB_VARIANT_TCGEN05_WIDE: case VXB_VARIANT_TCGEN05_WIDE_SILU: case VXB_VARIANT_GROUPED_TCGEN05: {
             if (id == VXB_VARIANT_GROUPED_TCGEN05) {
                 const GroupedFewShape few = grouped_few_shape(q.rows, q.n, (int)sms);   // few rows: weights as the M operand
                 if (few.slots) {
@@ -236,6 +240,9 @@ int vxb_plan(const VxbPlanQuery* query, VxbLaunchPlan* out, char* why, uint32_t 
             char unused[8];
             if (q.epilogue != VXB_EPI_I8 && round_up(q.k, kKAlign) <= VXB_WIDE_MAX_KPAD &&
                 admitted(kVariants[VXB_VARIANT_TCGEN05_WIDE], q, unused, sizeof unused)) chosen = VXB_VARIANT_TCGEN05_WIDE;
+            // ... and by the tail's arithmetic, from a full wave of tiles on
+            if ((q.fused_tail & 2u) && tiles >= sms && round_up(q.k, kKAlign) <= VXB_WIDE_MAX_KPAD &&
+                admitted(kVariants[VXB_VARIANT_TCGEN05_WIDE_SILU], q, unused, sizeof unused)) chosen = VXB_VARIANT_TCGEN05_WIDE_SILU;
         }
         if (!admitted(kVariants[chosen], q, why, why_bytes)) return 0;
     }
