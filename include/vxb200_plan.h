@@ -70,8 +70,8 @@ extern "C" {
     X(TCGEN05_WIDE,     8, "tcgen05-wide-i8",           "gemm_i8_wide_kernel",          128, 256, 128, 608, 1, 231000,   1,   0, 3u, 1u, 0, 1u | 4u | 32u, 640) \
     X(TCGEN05_WIDE_SILU, 0, "tcgen05-wide-silu-i8",    "gemm_i8_wide_kernel",          128, 256, 128, 608, 1, 231000,   1,   0, 2u, 1u, 0, 1u | 4u | 64u, 641) \
     X(GROUPED_TCGEN05,  0, "tcgen05-grouped-i8",        "gemm_i8_grouped_tcgen05_kernel", 128, 128, 128, 320, 1, 223000,   1,   0, 2u, 6u, 0, 1u,           500) \
-    X(GEMV_GROUPED,     0, "gemv-grouped",              "gemv_grouped_kernel",            0,   0,   0, 256, 1,  65536,   1,   4, 2u, 6u, 0, 1u,           550) \
-    X(GEMV_W4_GROUPED,  0, "gemv-w4-grouped",           "gemv_w4_grouped_kernel",         0,   0,   0, 256, 1,  65536,   1,   2, 2u, 4u, 0, 1u,           560) \
+    X(GEMV_GROUPED,     0, "gemv-grouped",              "gemv_grouped_kernel",            0,   0,   0, 256, 1, 147456,   1,   4, 2u, 6u, 0, 1u,           550) \
+    X(GEMV_W4_GROUPED,  0, "gemv-w4-grouped",           "gemv_w4_grouped_kernel",         0,   0,   0, 256, 1, 147456,   1,   2, 2u, 4u, 0, 1u,           560) \
     X(DP4A_GROUPED,     3, "dp4a-grouped",              "gemm_grouped_kernel",            4, 128,   0, 128, 1,      0,   1,   0, 2u, 6u, 0, 8u,             2)
 
 typedef enum VxbVariantId {

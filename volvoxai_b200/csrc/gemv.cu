@@ -181,6 +181,22 @@ gemm_grouped_kernel(const int8_t* __restrict__ q, uint32_t rows, const int8_t* _
 }
 
 
+// The weight ring of a warp: kRing steps of CH channels x 512 bytes, behind the staged activations.
+constexpr uint32_t kRing = 3;
+template <int CH> constexpr uint32_t kRingBytes = kGemvWarps * kRing * CH * 512u;   // of a CTA
+__device__ __forceinline__ void copy16_async(void* smem, const void* global, bool in) {
+    // bytes not read are zero-filled: a lane past the row's end or a channel past the last
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                 ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(global), "r"(in ? 16u : 0u) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void copy_wait_ahead() { asm volatile("cp.async.wait_group %0;" ::"n"(kRing - 1) : "memory"); }
+
+// f32(dot) * f32(as * ws): the exact fp32 value of |dot| < 2^22 without a conversion instruction, two rounded products
+__device__ __forceinline__ float group_product(int dot, float as, float gs) {
+    return __fmul_rn(__fadd_rn(__int_as_float(dot + 0x4B400000), -12582912.0f), __fmul_rn(as, gs));
+}
+
 // ---- grouped weight scales, few rows (decode) -------------------------------------------------
 // The reference's own decode mode: one row against PackedLinear storage with a scale per
 // G-element group.  Same streaming as gemv_dp4a_kernel (every warp reads CH weight rows with
@@ -188,9 +204,16 @@ gemm_grouped_kernel(const int8_t* __restrict__ q, uint32_t rows, const int8_t* _
 // but the integer partials are reduced only within the G/16 lanes that share a group, and after
 // every step the 512/G group dots go through the reference's arithmetic in ascending order:
 //   sum = sum + f32(dot_g) * f32(as * ws[n,g])        (every operation rounded on its own)
-// All lanes carry the same chain, so no lane diverges; int -> fp32 by the exact 1.5 * 2^23 trick.
+// Every lane turns the dot of its own group into that group's product (its scales arrive with the weights); the
+// products are then passed round in ascending order and all lanes carry the same chain of additions, so no lane
+// diverges; int -> fp32 by the exact 1.5 * 2^23 trick.
+// Bound by the weight stream: every lane copies its own 16 bytes per channel and step into shared memory
+// (cp.async, read back by the same lane, so no barrier), two steps ahead of the one it works on, and the first two
+// are requested before the launch in front of this one (the row quantizer) has finished.  In registers the same
+// depth took 80 to 100 of them, three CTAs per SM instead of four, and left a last wave of CTAs of its own: one row x
+// 4096 -> 14336 with its quantizer 15.5 us then and 13.4 now from int8, 14.9 and 11.8 from 4-bit words.
 template <int MR, int CH, int G>
-__global__ void __launch_bounds__(kGemvThreads)
+__global__ void __launch_bounds__(kGemvThreads, 4)
 gemv_grouped_kernel(const int8_t* __restrict__ q, uint32_t rows, const int8_t* __restrict__ w,
                     uint32_t n, uint32_t kpad, uint32_t kchunk, EpilogueParams epi) {
     extern __shared__ __align__(16) uint8_t smem[];  // [MR][kchunk] activations
@@ -200,8 +223,9 @@ gemv_grouped_kernel(const int8_t* __restrict__ q, uint32_t rows, const int8_t* _
     const uint32_t blocks = (n + kChannelsPerCta - 1) / kChannelsPerCta;
     const bool single_chunk = kchunk >= kpad;
     float as[MR];
-#pragma unroll
-    for (int m = 0; m < MR; m++) as[m] = (uint32_t)m < rows ? __ldg(epi.row_scales + m) : 0.0f;
+    bool waited = false;
+    pdl_release();
+    uint4* ring = reinterpret_cast<uint4*>(smem + (size_t)MR * kchunk) + warp * (kRing * CH * 32u) + lane;   // [kRing][CH][32 lanes]
 
     for (uint32_t blk = blockIdx.x; blk < blocks; blk += gridDim.x) {
         const uint32_t c0 = blk * kChannelsPerCta + warp * CH;
@@ -213,6 +237,30 @@ gemv_grouped_kernel(const int8_t* __restrict__ q, uint32_t rows, const int8_t* _
 
         for (uint32_t kb = 0; kb < kpad; kb += kchunk) {
             const uint32_t klen = kpad - kb < kchunk ? kpad - kb : kchunk;
+            // weights and scales of a step: a warp's K loop is otherwise a chain of load -> use round trips of a
+            // microsecond each
+            auto load_step = [&](uint32_t ks, uint32_t slot, float (&gr)[CH]) {
+                const uint32_t k = ks + lane * 16u, g = (kb + ks) / G + lane / kLanesPerGroup;
+#pragma unroll
+                for (int c = 0; c < CH; c++) {
+                    const uint32_t ch = c0 + c;
+                    const bool in = k < klen && ch < n;
+                    if (ks < klen) copy16_async(ring + (slot * CH + c) * 32u, w + (in ? (size_t)ch * kpad + kb + k : 0), in);
+                    gr[c] = (ks < klen && g < epi.groups && ch < n) ? __ldg(epi.gscales + (size_t)ch * epi.groups + g) : 0.0f;
+                }
+                copy_commit();
+            };
+            float gv[CH], g1[CH];
+            uint32_t slot = 0;
+            load_step(0, 0, gv);
+            load_step(512, 1, g1);
+            if (!waited) {
+                // what follows reads the preceding kernel's output, and its input may still be this one's output
+                pdl_wait();
+                waited = true;
+#pragma unroll
+                for (int m = 0; m < MR; m++) as[m] = (uint32_t)m < rows ? __ldg(epi.row_scales + m) : 0.0f;
+            }
             if (!(single_chunk && blk != blockIdx.x)) {
                 __syncthreads();
                 const uint32_t vec_per_row = klen / 16;
@@ -224,26 +272,15 @@ gemv_grouped_kernel(const int8_t* __restrict__ q, uint32_t rows, const int8_t* _
                 }
                 __syncthreads();
             }
-            // the next step's weights are requested before this step's arithmetic: a warp's K loop is
-            // otherwise a chain of load -> use round trips of a microsecond each
-            uint4 wv[CH];
-#pragma unroll
-            for (int c = 0; c < CH; c++) {
-                const uint32_t ch = c0 + c;
-                wv[c] = (lane * 16u < klen && ch < n) ? __ldcs(reinterpret_cast<const uint4*>(w + (size_t)ch * kpad + kb + lane * 16))
-                                                      : make_uint4(0, 0, 0, 0);
-            }
             for (uint32_t ks = 0; ks < klen; ks += 512) {
                 const uint32_t k0 = ks + lane * 16;
                 const bool in = k0 < klen;
-                int part[MR][CH];
-                uint4 wn[CH];
+                uint4 wv[CH];
+                float g2[CH], product[MR][CH];
+                load_step(ks + 1024u, slot == 0 ? kRing - 1 : slot - 1, g2);
+                copy_wait_ahead();
 #pragma unroll
-                for (int c = 0; c < CH; c++) {
-                    const uint32_t ch = c0 + c;
-                    wn[c] = (k0 + 512u < klen && ch < n) ? __ldcs(reinterpret_cast<const uint4*>(w + (size_t)ch * kpad + kb + k0 + 512u))
-                                                         : make_uint4(0, 0, 0, 0);
-                }
+                for (int c = 0; c < CH; c++) wv[c] = ring[(slot * CH + c) * 32u];
 #pragma unroll
                 for (int m = 0; m < MR; m++) {
                     const uint4 a = in ? *reinterpret_cast<const uint4*>(smem + (size_t)m * kchunk + k0) : make_uint4(0, 0, 0, 0);
@@ -255,7 +292,7 @@ gemv_grouped_kernel(const int8_t* __restrict__ q, uint32_t rows, const int8_t* _
                         s = dp4a_s8(a.w, wv[c].w, s);
 #pragma unroll
                         for (int off = kLanesPerGroup / 2; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-                        part[m][c] = s;
+                        product[m][c] = group_product(s, as[m], gv[c]);
                     }
                 }
                 const uint32_t g0 = (kb + ks) / G;
@@ -263,19 +300,13 @@ gemv_grouped_kernel(const int8_t* __restrict__ q, uint32_t rows, const int8_t* _
                 for (int j = 0; j < kGroupsPerStep; j++) {
                     if (g0 + j >= epi.groups) break;                       // uniform over the warp
 #pragma unroll
-                    for (int c = 0; c < CH; c++) {
-                        const uint32_t ch = c0 + c < n ? c0 + c : n - 1;
-                        const float gs = __ldg(epi.gscales + (size_t)ch * epi.groups + g0 + j);
+                    for (int c = 0; c < CH; c++)
 #pragma unroll
-                        for (int m = 0; m < MR; m++) {
-                            const int d = __shfl_sync(0xffffffffu, part[m][c], j * kLanesPerGroup);
-                            const float f = __fadd_rn(__int_as_float(d + 0x4B400000), -12582912.0f);
-                            sum[m][c] = __fadd_rn(sum[m][c], __fmul_rn(f, __fmul_rn(as[m], gs)));
-                        }
-                    }
+                        for (int m = 0; m < MR; m++) sum[m][c] = __fadd_rn(sum[m][c], __shfl_sync(0xffffffffu, product[m][c], j * kLanesPerGroup));
                 }
 #pragma unroll
-                for (int c = 0; c < CH; c++) wv[c] = wn[c];
+                for (int c = 0; c < CH; c++) { gv[c] = g1[c]; g1[c] = g2[c]; }
+                if (++slot == kRing) slot = 0;
             }
         }
 #pragma unroll
@@ -295,10 +326,9 @@ cudaError_t launch_gemv_grouped_t(const int8_t* q, uint32_t rows, const int8_t* 
                                   const EpilogueParams& epi, int sm_count, cudaStream_t stream) {
     const GemvShape shape = gemv_shape(1, rows, n, kpad, sm_count);
     if (shape.mr != (uint32_t)MR || shape.ch != (uint32_t)CH) return cudaErrorInvalidValue;
-    cudaError_t e = ensure_dynamic_smem<gemv_grouped_kernel<MR, CH, G>>(kGemvSmemBytes);
+    cudaError_t e = ensure_dynamic_smem<gemv_grouped_kernel<MR, CH, G>>(kGemvSmemBytes + kRingBytes<CH>);
     if (e != cudaSuccess) return e;
-    gemv_grouped_kernel<MR, CH, G><<<shape.grid, kGemvThreads, shape.smem, stream>>>(q, rows, w, n, kpad, shape.kchunk, epi);
-    return cudaGetLastError();
+    return launch_pdl(gemv_grouped_kernel<MR, CH, G>, dim3(shape.grid), dim3(kGemvThreads), shape.smem, stream, q, rows, w, n, kpad, shape.kchunk, epi);
 }
 
 template <int G>
@@ -319,7 +349,7 @@ cudaError_t launch_gemv_grouped_g(const int8_t* q, uint32_t rows, const int8_t* 
 // dp4a; sum a * (c - 8) = sum a * c - 8 * sum a, with sum a taken once per row and step.
 // Each lane owns 16 bytes = 32 codes of every 1024-code step; G / 32 lanes share a group.
 template <int MR, int CH, int G>
-__global__ void __launch_bounds__(kGemvThreads)
+__global__ void __launch_bounds__(kGemvThreads, 4)
 gemv_w4_grouped_kernel(const int8_t* __restrict__ q, uint32_t rows, const uint32_t* __restrict__ w4,
                        uint32_t row_words, uint32_t n, uint32_t kpad, uint32_t kchunk, EpilogueParams epi) {
     extern __shared__ __align__(16) uint8_t smem[];  // [MR][kchunk] de-interleaved activations
@@ -329,8 +359,9 @@ gemv_w4_grouped_kernel(const int8_t* __restrict__ q, uint32_t rows, const uint32
     const uint32_t blocks = (n + kChannelsPerCta - 1) / kChannelsPerCta;
     const bool single_chunk = kchunk >= kpad;
     float as[MR];
-#pragma unroll
-    for (int m = 0; m < MR; m++) as[m] = (uint32_t)m < rows ? __ldg(epi.row_scales + m) : 0.0f;
+    bool waited = false;
+    pdl_release();
+    uint4* ring = reinterpret_cast<uint4*>(smem + (size_t)MR * kchunk) + warp * (kRing * CH * 32u) + lane;   // [kRing][CH][32 lanes]
 
     for (uint32_t blk = blockIdx.x; blk < blocks; blk += gridDim.x) {
         const uint32_t c0 = blk * kChannelsPerCta + warp * CH;
@@ -342,6 +373,29 @@ gemv_w4_grouped_kernel(const int8_t* __restrict__ q, uint32_t rows, const uint32
 
         for (uint32_t kb = 0; kb < kpad; kb += kchunk) {
             const uint32_t klen = kpad - kb < kchunk ? kpad - kb : kchunk;
+            // (lanes past the row's end meet zero activations, so their weights do not matter)
+            auto load_step = [&](uint32_t ks, uint32_t slot, float (&gr)[CH]) {
+                const uint32_t k = ks + lane * 32u, g = (kb + ks) / G + lane / kLanesPerGroup;
+#pragma unroll
+                for (int c = 0; c < CH; c++) {
+                    const uint32_t ch = c0 + c;
+                    const bool in = k < klen && ch < n;
+                    if (ks < klen) copy16_async(ring + (slot * CH + c) * 32u, w4 + (in ? (size_t)ch * row_words + (kb + k) / 8 : 0), in);
+                    gr[c] = (ks < klen && g < epi.groups && ch < n) ? __ldg(epi.gscales + (size_t)ch * epi.groups + g) : 0.0f;
+                }
+                copy_commit();
+            };
+            float gv[CH], g1[CH];
+            uint32_t slot = 0;
+            load_step(0, 0, gv);
+            load_step(1024, 1, g1);
+            if (!waited) {
+                // what follows reads the preceding kernel's output, and its input may still be this one's output
+                pdl_wait();
+                waited = true;
+#pragma unroll
+                for (int m = 0; m < MR; m++) as[m] = (uint32_t)m < rows ? __ldg(epi.row_scales + m) : 0.0f;
+            }
             if (!(single_chunk && blk != blockIdx.x)) {
                 __syncthreads();
                 const uint32_t vec_per_row = klen / 16;
@@ -355,25 +409,15 @@ gemv_w4_grouped_kernel(const int8_t* __restrict__ q, uint32_t rows, const uint32
                 }
                 __syncthreads();
             }
-            const uint4 kZero4 = make_uint4(0x88888888u, 0x88888888u, 0x88888888u, 0x88888888u);
-            uint4 wv[CH];
-#pragma unroll
-            for (int c = 0; c < CH; c++) {
-                const uint32_t ch = c0 + c;
-                wv[c] = (lane * 32u < klen && ch < n) ? __ldcs(reinterpret_cast<const uint4*>(w4 + (size_t)ch * row_words + (kb + lane * 32u) / 8))
-                                                      : kZero4;
-            }
             for (uint32_t ks = 0; ks < klen; ks += 1024) {
                 const uint32_t k0 = ks + lane * 32;                  // this lane's first code of the step
                 const bool in = k0 < klen;
-                uint4 wn[CH];
+                uint4 wv[CH];
+                float g2[CH], product[MR][CH];
+                load_step(ks + 2048u, slot == 0 ? kRing - 1 : slot - 1, g2);
+                copy_wait_ahead();
 #pragma unroll
-                for (int c = 0; c < CH; c++) {
-                    const uint32_t ch = c0 + c;
-                    wn[c] = (k0 + 1024u < klen && ch < n) ? __ldcs(reinterpret_cast<const uint4*>(w4 + (size_t)ch * row_words + (kb + k0 + 1024u) / 8))
-                                                          : kZero4;
-                }
-                int part[MR][CH];
+                for (int c = 0; c < CH; c++) wv[c] = ring[(slot * CH + c) * 32u];
 #pragma unroll
                 for (int m = 0; m < MR; m++) {
                     uint4 a0 = make_uint4(0, 0, 0, 0), a1 = a0;
@@ -397,7 +441,7 @@ gemv_w4_grouped_kernel(const int8_t* __restrict__ q, uint32_t rows, const uint32
                         s -= 8 * asum;
 #pragma unroll
                         for (int off = kLanesPerGroup / 2; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-                        part[m][c] = s;
+                        product[m][c] = group_product(s, as[m], gv[c]);
                     }
                 }
                 const uint32_t g0 = (kb + ks) / G;
@@ -405,19 +449,13 @@ gemv_w4_grouped_kernel(const int8_t* __restrict__ q, uint32_t rows, const uint32
                 for (int j = 0; j < kGroupsPerStep; j++) {
                     if (g0 + j >= epi.groups) break;                       // uniform over the warp
 #pragma unroll
-                    for (int c = 0; c < CH; c++) {
-                        const uint32_t ch = c0 + c < n ? c0 + c : n - 1;
-                        const float gs = __ldg(epi.gscales + (size_t)ch * epi.groups + g0 + j);
+                    for (int c = 0; c < CH; c++)
 #pragma unroll
-                        for (int m = 0; m < MR; m++) {
-                            const int d = __shfl_sync(0xffffffffu, part[m][c], j * kLanesPerGroup);
-                            const float f = __fadd_rn(__int_as_float(d + 0x4B400000), -12582912.0f);
-                            sum[m][c] = __fadd_rn(sum[m][c], __fmul_rn(f, __fmul_rn(as[m], gs)));
-                        }
-                    }
+                        for (int m = 0; m < MR; m++) sum[m][c] = __fadd_rn(sum[m][c], __shfl_sync(0xffffffffu, product[m][c], j * kLanesPerGroup));
                 }
 #pragma unroll
-                for (int c = 0; c < CH; c++) wv[c] = wn[c];
+                for (int c = 0; c < CH; c++) { gv[c] = g1[c]; g1[c] = g2[c]; }
+                if (++slot == kRing) slot = 0;
             }
         }
 #pragma unroll
@@ -437,10 +475,9 @@ cudaError_t launch_gemv_w4_t(const int8_t* q, uint32_t rows, const uint32_t* w4,
                              uint32_t kpad, const EpilogueParams& epi, int sm_count, cudaStream_t stream) {
     const GemvShape shape = gemv_shape(2, rows, n, kpad, sm_count);
     if (shape.mr != (uint32_t)MR || shape.ch != (uint32_t)CH) return cudaErrorInvalidValue;
-    cudaError_t e = ensure_dynamic_smem<gemv_w4_grouped_kernel<MR, CH, G>>(kGemvSmemBytes);
+    cudaError_t e = ensure_dynamic_smem<gemv_w4_grouped_kernel<MR, CH, G>>(kGemvSmemBytes + kRingBytes<CH>);
     if (e != cudaSuccess) return e;
-    gemv_w4_grouped_kernel<MR, CH, G><<<shape.grid, kGemvThreads, shape.smem, stream>>>(q, rows, w4, row_words, n, kpad, shape.kchunk, epi);
-    return cudaGetLastError();
+    return launch_pdl(gemv_w4_grouped_kernel<MR, CH, G>, dim3(shape.grid), dim3(kGemvThreads), shape.smem, stream, q, rows, w4, row_words, n, kpad, shape.kchunk, epi);
 }
 
 template <int G>
@@ -470,10 +507,11 @@ GemvShape gemv_shape(int kind, uint32_t rows, uint32_t n, uint32_t kpad, int sm_
     const uint32_t step = kind == 2 ? 1024u : 512u;
     s.kchunk = kind == 0 ? kpad : (kpad + step - 1) / step * step;
     if ((uint64_t)s.mr * s.kchunk > kGemvSmemBytes) s.kchunk = (kGemvSmemBytes / s.mr) / step * step;
-    s.smem = s.mr * s.kchunk;
+    const uint32_t ring = kind == 0 ? 0u : (uint32_t)kGemvWarps * kRing * s.ch * 512u;   // the grouped kernels' weight rings
+    s.smem = s.mr * s.kchunk + ring;
     const uint32_t per_cta = (uint32_t)kGemvWarps * s.ch;
     const uint32_t blocks = (n + per_cta - 1) / per_cta;
-    uint32_t per_sm = s.smem ? (200u * 1024u) / (s.smem + 1024u) : 8u;
+    uint32_t per_sm = s.smem ? (kind == 0 ? 200u * 1024u : 227u * 1024u) / (s.smem + 1024u) : 8u;
     if (per_sm > 8) per_sm = 8;
     if (per_sm < 1) per_sm = 1;
     s.grid = (uint32_t)sm_count * per_sm;
