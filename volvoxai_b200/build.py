@@ -56,6 +56,31 @@ def build(force: bool = False, verbose: bool = False) -> str:
     return LIB
 
 
+TORCH_CALLS = os.path.join(PKG, "_torch_calls.so")
+TORCH_CALLS_SRC = os.path.join(CSRC, "torch_calls.cpp")
+
+
+def build_torch_calls(force: bool = False) -> str:
+    """Builds _torch_calls.so (w8a8.py's device calls in native code) against the running Python's torch."""
+    deps = [TORCH_CALLS_SRC, os.path.join(ROOT, "include", "vxb200_w8a8.h")]
+    if not force and os.path.exists(TORCH_CALLS) and all(os.path.getmtime(d) <= os.path.getmtime(TORCH_CALLS) for d in deps):
+        return TORCH_CALLS
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+    includes = [f"-isystem{p}" for p in cpp_extension.include_paths() + [sysconfig.get_paths()["include"]]]
+    torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cmd = ["g++", "-std=c++20", "-O2", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+           *includes, "-o", TORCH_CALLS, TORCH_CALLS_SRC, "-L", PKG, "-l:libvxb200.so", "-Wl,-rpath,$ORIGIN",
+           "-L", torch_lib, "-lc10", "-ltorch_cpu", "-ltorch_python"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        sys.stderr.write(res.stdout + res.stderr)
+        raise RuntimeError("g++ failed building _torch_calls.so")
+    return TORCH_CALLS
+
+
 PROVIDER_LIB = os.path.join(PKG, "libvxb200_provider.so")
 PROVIDER_SRC = os.path.join(PKG, "provider", "vxb200_provider.c")
 
@@ -89,4 +114,5 @@ def build_provider(force: bool = False) -> str | None:
 if __name__ == "__main__":
     build(force="--force" in sys.argv, verbose="-v" in sys.argv or "--force" in sys.argv)
     print(LIB)
+    print(build_torch_calls(force="--force" in sys.argv))
     print(build_provider(force="--force" in sys.argv))

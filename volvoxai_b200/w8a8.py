@@ -50,6 +50,29 @@ def _ptr(a) -> C.c_void_p:
     return C.c_void_p(a.data_ptr())  # torch tensor
 
 
+_torch_calls = False   # not looked for yet
+
+
+def _calls(x):
+    """The native form of the device calls (csrc/torch_calls.cpp) for a torch tensor; None for anything else, or where
+    the module was not built: the ctypes form below serves then, with the same results."""
+    global _torch_calls
+    if _torch_calls is False:
+        try:
+            import torch
+            from . import _torch_calls as module
+            _torch_calls = (module, torch.Tensor)
+        except ImportError:
+            _torch_calls = None
+    return _torch_calls[0] if _torch_calls is not None and isinstance(x, _torch_calls[1]) else None
+
+
+def _done(result):
+    if result.__class__ is int:
+        raise W8A8Error(result)
+    return result
+
+
 def launch_count() -> int:
     return int(_lib.load().vxb_launch_count())
 
@@ -115,6 +138,7 @@ class Context:
         h = C.c_void_p(0)
         _check(self._L.vxb_context_create(device, C.c_void_p(stream or 0), C.byref(h)))
         self.handle = h
+        self._h = h.value
 
     def set_stream(self, stream: int | None) -> None:
         _check(self._L.vxb_context_set_stream(self.handle, C.c_void_p(stream or 0)))
@@ -175,6 +199,7 @@ class Context:
         if getattr(self, "handle", None):
             self._L.vxb_context_destroy(self.handle)
             self.handle = None
+            self._h = 0
 
     def __del__(self):
         try:
@@ -211,9 +236,12 @@ class Context:
     def rmsnorm_linear_f32_fused(self, w: "Weight", x, norm_weight, epsilon: float, silu_mul: bool = False,
                                  norm_out=None, out=None):
         """RMSNorm -> quantize -> linear (+ silu(gate) * up over interleaved channel pairs)."""
+        width = w.d_out // 2 if silu_mul else w.d_out
+        native = _calls(x)
+        if native is not None:
+            return _done(native.rmsnorm_linear_f32_fused(self._h, w._h, x, width, out, norm_weight, epsilon, norm_out, 1 if silu_mul else 0))
         import torch
         rows = x.shape[0]
-        width = w.d_out // 2 if silu_mul else w.d_out
         if out is None:
             out = torch.empty((rows, width), dtype=torch.float32, device=x.device)
         _check(self._L.vxb_rmsnorm_linear_f32_fused(self.handle, w.handle, _ptr(x), _ptr(norm_weight), float(epsilon),
@@ -222,6 +250,9 @@ class Context:
         return out
 
     def linear_f32(self, w: "Weight", x, out=None, route: int = ROUTE_AUTO):
+        native = _calls(x)
+        if native is not None:
+            return _done(native.linear_f32(self._h, w._h, x, w.d_out, out, route))
         import torch
         rows = x.shape[0]
         if out is None:
@@ -233,9 +264,12 @@ class Context:
     def linear_f32_fused(self, w: "Weight", x, residual=None, silu_mul: bool = False, out=None):
         """fp32 linear with a fused tail: + residual, or silu(gate) * up over interleaved channel
         pairs (output d_out / 2 wide)."""
+        width = w.d_out // 2 if silu_mul else w.d_out
+        native = _calls(x)
+        if native is not None:
+            return _done(native.linear_f32_fused(self._h, w._h, x, width, out, residual, 1 if silu_mul else 0))
         import torch
         rows = x.shape[0]
-        width = w.d_out // 2 if silu_mul else w.d_out
         if out is None:
             out = torch.empty((rows, width), dtype=torch.float32, device=x.device)
         _check(self._L.vxb_linear_f32_fused(self.handle, w.handle, _ptr(x), rows, _ptr(out), out.stride(0),
@@ -246,6 +280,9 @@ class Context:
 
     def linear_i8(self, w: "Weight", x, out_scale: float, out_zero: int = 0, out=None,
                   route: int = ROUTE_AUTO):
+        native = _calls(x)
+        if native is not None:
+            return _done(native.linear_i8(self._h, w._h, x, w.d_out, out, out_scale, int(out_zero), route))
         import torch
         rows = x.shape[0]
         if out is None:
@@ -279,6 +316,9 @@ class Context:
 
     # ---- boundary of a static W8A8 island (torch CUDA tensors) ----
     def quantize_linear(self, x, scale: float, zero_point: int = 0, unsigned: bool = False):
+        native = _calls(x)
+        if native is not None:
+            return _done(native.quantize_linear(self._h, x, scale, int(zero_point), 1 if unsigned else 0))
         import torch
         out = torch.empty(x.shape, dtype=torch.uint8 if unsigned else torch.int8, device=x.device)
         _check(self._L.vxb_quantize_linear_device(self.handle, _ptr(x), x.numel(), float(scale), int(zero_point),
@@ -286,6 +326,9 @@ class Context:
         return out
 
     def dequantize_linear(self, x, scale: float, zero_point: int = 0):
+        native = _calls(x)
+        if native is not None:
+            return _done(native.dequantize_linear(self._h, x, scale, int(zero_point)))
         import torch
         out = torch.empty(x.shape, dtype=torch.float32, device=x.device)
         _check(self._L.vxb_dequantize_linear_device(self.handle, _ptr(x), x.numel(), float(scale), int(zero_point),
@@ -294,6 +337,10 @@ class Context:
 
     def requantize_linear(self, x, input_scale: float, input_zero_point: int, output_scale: float,
                           output_zero_point: int, unsigned: bool = False):
+        native = _calls(x)
+        if native is not None:
+            return _done(native.requantize_linear(self._h, x, input_scale, int(input_zero_point), output_scale,
+                                                  int(output_zero_point), 1 if unsigned else 0))
         import torch
         out = torch.empty(x.shape, dtype=torch.uint8 if unsigned else torch.int8, device=x.device)
         _check(self._L.vxb_requantize_linear_device(self.handle, _ptr(x), x.numel(), float(input_scale),
@@ -304,6 +351,10 @@ class Context:
 
     def qlinear_device(self, w: "Weight", x, input_scale, input_zero, output_scale, output_zero,
                        out_unsigned: bool = False, route: int = ROUTE_AUTO):
+        native = _calls(x)
+        if native is not None:
+            return _done(native.qlinear_device(self._h, w._h, x, w.d_out, input_scale, int(input_zero), output_scale,
+                                               int(output_zero), 1 if out_unsigned else 0, route))
         import torch
         rows = x.shape[0]
         in_dt = DT_U8 if x.dtype == torch.uint8 else DT_I8
@@ -323,6 +374,7 @@ class Weight:
         self._L = ctx._L
         self.ctx = ctx
         self.handle = handle
+        self._h = handle.value
         self.d_in = int(self._L.vxb_weight_d_in(handle))
         self.d_out = int(self._L.vxb_weight_d_out(handle))
         self.row_bytes = int(self._L.vxb_weight_row_bytes(handle))
@@ -372,6 +424,7 @@ class Weight:
         if getattr(self, "handle", None):
             self._L.vxb_weight_destroy(self.handle)
             self.handle = None
+            self._h = 0
 
     def __del__(self):
         try:
