@@ -57,6 +57,8 @@ extern "C" {
  *   (0 = ceil(d_out / SMs) whole channels per CTA), tile K bytes, threads per CTA, CTAs per cluster,
  *   dynamic shared memory bound in bytes, minimum rows, maximum rows (0 = unbounded),
  *   epilogue mask, weight-kind mask, required group size (0 = any), flags, registry priority.
+ * GROUPED_TCGEN05 up to 64 rows launches gemm_i8_grouped_few_kernel (weights as the M operand); the plan's tile, threads
+ * and grid are that kernel's then.
  */
 #define VXB_VARIANTS(X) \
     X(DECODE_ROWS,      4, "decode-rows-tcgen05-i8",    "decode_rows_kernel",             0,   0, 128, 544, 1, 204800,   1, 128, 7u, 1u, 0, 1u | 4u,      700) \

@@ -185,6 +185,7 @@ struct VxbWeight {
     CUtensorMap tmap_w128;     // box 128 rows (stream-K decode kernel, pairs of CTAs)
     CUtensorMap tmap_w64;      // box 64 rows (pairs of CTAs on narrow tiles)
     CUtensorMap tmap_rows;     // box tile_rows rows (channel-owning decode kernel)
+    CUtensorMap tmap_few;      // box of two K blocks x the few-row kernel's channels (grouped scales)
     uint32_t tile_rows = 0, tiles_per_cta = 0;
     bool has_tmap = false;
     uint64_t bytes = 0;
@@ -262,7 +263,8 @@ int finish_weight(VxbContext* ctx, VxbWeight* w, const uint8_t* staging, uint32_
                   encode_i8_rows(&w->tmap_w128, w->w, n, w->kpad, 128) &&
                   encode_i8_rows(&w->tmap_w64, w->w, n, w->kpad, 64);
     decode_rows_plan(n, ctx->sm_count, &w->tile_rows, &w->tiles_per_cta);
-    w->has_tmap = w->has_tmap && encode_i8_rows(&w->tmap_rows, w->w, n, w->kpad, w->tile_rows);
+    w->has_tmap = w->has_tmap && encode_i8_rows(&w->tmap_rows, w->w, n, w->kpad, w->tile_rows) &&
+                  encode_i8_kblocks(&w->tmap_few, w->w, n, w->kpad, grouped_few_shape(1, n, ctx->sm_count).channels, 2);
     CUDA_TRY(cudaStreamSynchronize(ctx->stream), -1);
     return 1;
 }
@@ -390,11 +392,10 @@ int run_gemm(VxbContext* ctx, const VxbWeight* w, const int8_t* q, uint32_t rows
             }
             GemmGroupedArgs a;
             const GroupedFewShape few = grouped_few_shape(rows, w->d_out, ctx->sm_count);
-            if (few.slots ? !(encode_i8_kblocks(&a.tmap_a, q, rows, w->kpad, few.slots, 2) &&
-                              encode_i8_kblocks(&a.tmap_b, w->w, w->d_out, w->kpad, few.channels, 2))
-                          : !encode_i8_rows(&a.tmap_a, q, rows, w->kpad, 128))
+            if (!(few.slots ? encode_i8_kblocks(&a.tmap_a, q, rows, w->kpad, few.slots, 2)
+                            : encode_i8_rows(&a.tmap_a, q, rows, w->kpad, 128)))
                 return fail(0, "cuTensorMapEncodeTiled failed for activations");
-            if (!few.slots) a.tmap_b = w->tmap_w128;
+            a.tmap_b = few.slots ? w->tmap_few : w->tmap_w128;
             a.rows = rows; a.n = w->d_out; a.kpad = w->kpad;
             a.group = w->group; a.groups = w->groups; a.n_pad = w->n_pad; a.gscales_t = w->gscales_t;
             a.row_scales = epi.row_scales; a.bias = epi.bias_f32; a.out = (float*)epi.out; a.ld = epi.ld;

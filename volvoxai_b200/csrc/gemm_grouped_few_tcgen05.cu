@@ -7,17 +7,17 @@
 // the N operand (16 .. 64 columns; up to 8 tokens only the first 8 are drained), so that every lane of every drain warp owns a channel and a group costs a warp
 // five instructions per token.  With the tokens as M (the large kernel), 8 tokens left two of eight warps to drain
 // 128 columns for 32 lanes, 24 of them dead, group after group.  Whole call, quantizer included, G = 128: 8 x 4096 ->
-// 14336 14.3 us (30.8 before; the weights alone take 9.0 at the measured copy rate), 8 x 4096 -> 4096 13.8 (27.3),
-// 64 x 4096 -> 14336 17.9 (28.2).
+// 14336 15.5 us (30.8 before, both without what Python adds; the weights alone take 9.0 at the measured copy rate),
+// 8 x 4096 -> 4096 9.7 (27.3), 64 x 4096 -> 14336 18.9 (28.2).
 //
 // A stage is 256 bytes of K: one TMA box of weights ([2 K blocks][channels x 128 B]), one of activations, one commit,
-// and the 1 .. 8 groups that lie in it, each in accumulator columns of its own, drained together.  The ring holds
-// about 200 KB per SM, which is what keeps the HBM stream going.
+// and the 1 .. 8 groups that lie in it, each in accumulator columns of its own, drained together.  The rings hold about
+// 200 KB per SM, which is what keeps the HBM stream going.
 //
 //   warp 0        TMA producer, activations (waits for the launch before this one)
-//   warp 1        allocates TMEM; one lane issues the MMAs
+//   warp 1        allocates TMEM; one lane issues the MMAs (of the short tiles every other stage's; another warp the rest)
 //   warps 2..     drain: one per TMEM lane quarter (two for 64 tokens, 32 tokens each)
-//   last warp     TMA producer, weights (waits for nothing)
+//   next warp     TMA producer, weights (waits for nothing)
 //
 // Channels per tile: 128; 64 where the tiles of 128 would leave half of the SMs without one (an MMA takes its 128 or 64
 // clocks whatever the token count, so a tile of 128 channels and K = 4096 is 8.6 us of tensor pipe, of 64 half that).
@@ -32,29 +32,40 @@ namespace {
 using namespace tc;
 
 constexpr uint32_t kSpan = 128, kSpans = 2;   // K bytes of a swizzle span, spans per stage
-constexpr uint32_t kTmemCols = 512;
-constexpr uint32_t kSmemBudget = 216 * 1024;
 constexpr uint32_t kMaxStages = 12, kMaxBufs = 4;
 
 // BM channels per tile, LT live token slots, MPG MMAs (32 bytes of K) per group
 template <uint32_t BM, uint32_t LT, uint32_t MPG> struct Few {
     static constexpr uint32_t NT = LT < 16 ? 16 : LT;               // token columns of the MMA
+    // Up to 16 tokens two CTAs fit an SM (half of its shared memory and TMEM each), so that the next launch's CTAs
+    // start their weights while this launch drains: 8 x 4096 -> 14336 17.3 -> 16.5 us.  The short tiles want the deep
+    // ring instead (8 x 4096 -> 4096 13.7 us, 14.6 with half of it).
+    static constexpr bool kTwo = BM == 128 && LT <= 16;
+    static constexpr uint32_t kCtas = kTwo ? 2 : 1, kTmemCols = kTwo ? 256 : 512, kSmemBudget = (kTwo ? 110 : 216) * 1024;
     static constexpr uint32_t kDrainWarps = NT == 64 ? 8 : 4;
     static constexpr uint32_t kTokens = LT * 4 / kDrainWarps;       // tokens per drain thread
-    static constexpr uint32_t kWWarp = 2 + kDrainWarps;
-    static constexpr uint32_t kThreads = 32 * (kWWarp + 1);
     static constexpr uint32_t kWBytes = kSpans * BM * kSpan, kXBytes = kSpans * NT * kSpan, kStageBytes = kWBytes + kXBytes;
     static constexpr uint32_t kGroups = 8 / MPG;                    // groups per stage
+    // Stages whose scales are requested ahead: a stage of 64 channels lasts 0.3 us, of 128 twice that, a scale from memory
+    // up to one (8 x 14336 -> 4096: 40.1 us one stage ahead, 23.6 four ahead; 8 x 4096 -> 14336 16.4, 15.5).  Where a
+    // stage is long and its drain is too (64 tokens 18.9 us, 20.3 four ahead; eight groups 18.8, 19.7) one is enough.
+    static constexpr uint32_t kAhead = BM == 64 ? (kGroups >= 8 ? 2 : 4) : LT <= 8 && kGroups <= 4 ? 4 : 1;
     static constexpr uint32_t kAccCols = NT * kGroups;
     static constexpr uint32_t kBufs = kTmemCols / kAccCols < kMaxBufs ? kTmemCols / kAccCols : kMaxBufs;
+    // Short tiles: two threads issue, stage by stage in turn (a thread starts an MMA every hundred clocks or so, and
+    // one of 64 rows is done in 64).  Stages and accumulators then come in even numbers, so that each belongs to one
+    // of them: a parity wait means something only to a waiter that saw the phase before.
+    static constexpr uint32_t kIssuers = BM == 64 && kBufs % 2 == 0 ? 2 : 1;
+    static constexpr uint32_t kWWarp = 2 + kDrainWarps;
+    static constexpr uint32_t kThreads = 32 * (kWWarp + kIssuers);  // the second issuer is the last warp
     static constexpr uint32_t kFit = kSmemBudget / kStageBytes;
-    static constexpr uint32_t kStages = kFit < kMaxStages ? kFit : kMaxStages;
+    static constexpr uint32_t kStages = (kFit < kMaxStages ? kFit : kMaxStages) / kIssuers * kIssuers;
     static constexpr uint32_t kOffBars = kStages * kStageBytes;
     static constexpr uint32_t kNumBars = 2 * kStages + 2 * kBufs;
     static constexpr uint32_t kOffTmemPtr = kOffBars + kNumBars * 8;
     static constexpr uint32_t kOffAbort = kOffTmemPtr + 4;
     static constexpr uint32_t kSmemBytes = kOffAbort + 8 + 1024;
-    static_assert(kSmemBytes <= 227 * 1024 && kStages >= 2 && kBufs >= 1, "launch shape");
+    static_assert(kSmemBytes <= 227 * 1024 && kStages >= 2 && kBufs >= 1 && kStages % kIssuers == 0, "launch shape");
 };
 
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
@@ -67,7 +78,7 @@ __device__ __forceinline__ void tmem_ld_tokens(uint32_t taddr, uint32_t (&r)[16]
 __device__ __forceinline__ void tmem_ld_tokens(uint32_t taddr, uint32_t (&r)[32]) { tmem_ld32(taddr, r); }
 
 template <uint32_t BM, uint32_t LT, uint32_t MPG>
-__global__ void __launch_bounds__(Few<BM, LT, MPG>::kThreads, 1)
+__global__ void __launch_bounds__(Few<BM, LT, MPG>::kThreads, Few<BM, LT, MPG>::kCtas)
 gemm_i8_grouped_few_kernel(const __grid_constant__ GemmGroupedArgs args) {
     using C = Few<BM, LT, MPG>;
     constexpr uint32_t NT = C::NT;
@@ -97,7 +108,7 @@ gemm_i8_grouped_few_kernel(const __grid_constant__ GemmGroupedArgs args) {
         pdl_release();   // the next launch in the stream may begin its own prologue
     }
     if (warp == 1) {
-        tmem_alloc(smem_u32(tmem_ptr), kTmemCols);
+        tmem_alloc(smem_u32(tmem_ptr), C::kTmemCols);
         tmem_relinquish();
     }
     tc_fence_before();
@@ -137,31 +148,32 @@ gemm_i8_grouped_few_kernel(const __grid_constant__ GemmGroupedArgs args) {
                 }
             }
         }
-    } else if (warp == 1) {
-        // ---------------- MMA issuer ----------------
+    } else if (warp == 1 || warp > C::kWWarp) {
+        // ---------------- MMA issuers: stages `me`, me + kIssuers, ... of this CTA's ----------------
         if (lane == 0) {
             constexpr uint32_t idesc = make_idesc(BM, NT);
-            uint32_t stage = 0, phase = 0, buf = 0, buf_phase = 0;
-            bool ok = true;
-            for (uint32_t t = blockIdx.x; ok && t < tiles; t += gridDim.x) {
-                for (uint32_t kb = 0; kb < num_kb; kb++) {
-                    if (!mbar_wait(tmem_empty(buf), buf_phase ^ 1u, abort_flag)) { ok = false; break; }
-                    if (!mbar_try_wait(full(stage), phase) && !mbar_wait(full(stage), phase, abort_flag)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint32_t w_lo = smem_desc_lo(w_addr(stage)), x_lo = smem_desc_lo(w_addr(stage) + C::kWBytes);
-                    const uint32_t left = total_ks - kb * 8u;
+            const uint32_t me = warp == 1 ? 0u : 1u;
+            uint32_t stage = me, phase = 0, buf = me, buf_phase = 0, kb = me;
+            for (uint32_t t = blockIdx.x;;) {
+                while (kb >= num_kb) { kb -= num_kb; t += gridDim.x; }
+                if (t >= tiles) break;
+                if (!mbar_wait(tmem_empty(buf), buf_phase ^ 1u, abort_flag)) break;
+                if (!mbar_try_wait(full(stage), phase) && !mbar_wait(full(stage), phase, abort_flag)) break;
+                tc_fence_after();
+                const uint32_t w_lo = smem_desc_lo(w_addr(stage)), x_lo = smem_desc_lo(w_addr(stage) + C::kWBytes);
+                const uint32_t left = total_ks - kb * 8u;
 #pragma unroll
-                    for (uint32_t j = 0; j < 8; j++) {
-                        if (j >= left) break;
-                        const uint32_t span = j >> 2, in = 2u * (j & 3u);    // +32 bytes of K = +2
-                        umma_i8_lo_first(tmem_base + buf * C::kAccCols + (j / MPG) * NT, w_lo + span * (BM * kSpan >> 4) + in,
-                                         x_lo + span * (NT * kSpan >> 4) + in, idesc, j % MPG);
-                    }
-                    umma_commit(empty(stage));
-                    umma_commit(tmem_full(buf));
-                    if (++stage == C::kStages) { stage = 0; phase ^= 1u; }
-                    if (++buf == C::kBufs) { buf = 0; buf_phase ^= 1u; }
+                for (uint32_t j = 0; j < 8; j++) {
+                    if (j >= left) break;
+                    const uint32_t span = j >> 2, in = 2u * (j & 3u);    // +32 bytes of K = +2
+                    umma_i8_lo_first(tmem_base + buf * C::kAccCols + (j / MPG) * NT, w_lo + span * (BM * kSpan >> 4) + in,
+                                     x_lo + span * (NT * kSpan >> 4) + in, idesc, j % MPG);
                 }
+                umma_commit(empty(stage));
+                umma_commit(tmem_full(buf));
+                kb += C::kIssuers;
+                if ((stage += C::kIssuers) >= C::kStages) { stage = me; phase ^= 1u; }
+                if ((buf += C::kIssuers) >= C::kBufs) { buf = me; buf_phase ^= 1u; }
             }
         }
     } else {
@@ -183,19 +195,26 @@ gemm_i8_grouped_few_kernel(const __grid_constant__ GemmGroupedArgs args) {
             float sum[C::kTokens];
 #pragma unroll
             for (uint32_t i = 0; i < C::kTokens; i++) sum[i] = 0.0f;
-            // the scales of the next stage's groups are on their way while this stage's are used
-            float next[C::kGroups];
+            // the scales of the next kAhead stages' groups are on their way while this stage's are used
+            float ahead[C::kAhead][C::kGroups];
 #pragma unroll
-            for (uint32_t g = 0; g < C::kGroups; g++) next[g] = g < args.groups ? __ldg(gs + (size_t)g * args.n_pad) : 0.0f;
+            for (uint32_t u = 0; u < C::kAhead; u++)
+#pragma unroll
+                for (uint32_t g = 0; g < C::kGroups; g++)
+                    ahead[u][g] = u * C::kGroups + g < args.groups ? __ldg(gs + (size_t)(u * C::kGroups + g) * args.n_pad) : 0.0f;
 #pragma unroll 1
-            for (uint32_t kb = 0; kb < num_kb; kb++) {
+            for (uint32_t kb0 = 0; ok && kb0 < num_kb; kb0 += C::kAhead)
+#pragma unroll
+            for (uint32_t u = 0; u < C::kAhead; u++) {
+                const uint32_t kb = kb0 + u;
+                if (kb >= num_kb) break;
                 const uint32_t g0 = kb * C::kGroups;
                 float cur[C::kGroups];
 #pragma unroll
                 for (uint32_t g = 0; g < C::kGroups; g++) {
-                    cur[g] = next[g];
-                    const uint32_t ng = g0 + C::kGroups + g;
-                    next[g] = ng < args.groups ? __ldg(gs + (size_t)ng * args.n_pad) : 0.0f;
+                    cur[g] = ahead[u][g];
+                    const uint32_t ng = g0 + C::kAhead * C::kGroups + g;
+                    ahead[u][g] = ng < args.groups ? __ldg(gs + (size_t)ng * args.n_pad) : 0.0f;
                 }
                 ok = __all_sync(0xffffffffu, mbar_wait(tmem_full(buf), buf_phase, abort_flag));
                 if (!ok) break;
@@ -239,7 +258,7 @@ gemm_i8_grouped_few_kernel(const __grid_constant__ GemmGroupedArgs args) {
         __syncthreads();
     }
     tc_fence_after();
-    if (warp == 1) tmem_dealloc(tmem_base, kTmemCols);
+    if (warp == 1) tmem_dealloc(tmem_base, C::kTmemCols);
 }
 
 template <uint32_t BM, uint32_t LT, uint32_t MPG>
@@ -279,7 +298,7 @@ GroupedFewShape grouped_few_shape(uint32_t rows, uint32_t n, int sm_count) {
     s.channels = 2u * ((n + 127u) / 128u) <= (uint32_t)sm_count ? 64u : 128u;
     const uint32_t tiles = (n + s.channels - 1) / s.channels;
     s.grid = tiles < (uint32_t)sm_count ? tiles : (uint32_t)sm_count;
-    s.threads = s.slots == 64 ? 352u : 224u;
+    s.threads = (s.slots == 64 ? 352u : 224u) + (s.channels == 64 ? 32u : 0u);   // (a second issuer)
     return s;
 }
 
