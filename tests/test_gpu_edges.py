@@ -206,3 +206,20 @@ def test_rmsnorm_products_near_and_far_from_one(torch, ctx, rows, k):
     y = y.cpu().numpy()
     # one rounding to fp32 each; a 64-bit rounding can tip it in a handful of elements, by one place
     assert (np.abs(y.view(np.int32).astype(np.int64) - want.view(np.int32)) <= 1).all() and (y != want).mean() <= 1e-4
+
+
+@pytest.mark.parametrize("rows,k,n", [(65, 1024, 3080), (100, 1152, 200), (128, 4096, 1000), (66, 64, 4000)])
+def test_rows_past_64_in_tiles(torch, ctx, rows, k, n):
+    """65 to 128 rows outside the small weights take the tile kernels: every output equal to the decode kernel's."""
+    from volvoxai_b200 import w8a8
+    c = wl.single_linear(rows=rows, k=k, n=n, seed=rows + k + n)
+    weight = w8a8.Weight.from_i8(ctx, c["w"], c["ws"], bias_f32=c["bias"], bias_i32=np.arange(n, dtype=np.int32) * 5 - 300)
+    x = dev(torch, c["x"])
+    res = torch.randn((rows, n), device="cuda")
+    for call in (lambda r: ctx.linear_acc_i32(weight, x, route=r), lambda r: ctx.linear_f32(weight, x, route=r),
+                 lambda r: ctx.linear_i8(weight, x, 0.1, -5, route=r)):
+        y = call(w8a8.ROUTE_AUTO)
+        assert "tcgen05" in w8a8.last_route() and "decode" not in w8a8.last_route()
+        assert torch.equal(y, call(w8a8.ROUTE_DECODE))
+    assert torch.equal(ctx.linear_f32_fused(weight, x, residual=res), ctx.linear_f32(weight, x, route=w8a8.ROUTE_DECODE) + res)
+    weight.close()

@@ -209,7 +209,10 @@ int vxb_plan(const VxbPlanQuery* query, VxbLaunchPlan* out, char* why, uint32_t 
             if (q.rows > 128 && tiles >= 2u * sms && (uint64_t)q.n_peers * 3424u <= round_up(q.k, kKAlign) &&
                 admitted(kVariants[VXB_VARIANT_TCGEN05_PAIR], q, unused, sizeof unused)) chosen = VXB_VARIANT_TCGEN05_PAIR;
         }
-        else if (q.rows <= 128) {
+        else if (q.rows <= 64 || (q.rows <= 128 && round_up(q.k, kKAlign) <= 1024u && q.n <= 3072u)) {
+            // (65 to 128 rows are 128 token slots, and an MMA of the decode kernel takes its 128 clocks whatever its
+            // channels: 128 x 4096 -> 4096 20.9 us against 16.2 in tiles of 128 x 256, 128 x 1024 -> 6144 13.3 against
+            // 9.1, 128 x 1024 -> 3072 9.5 against 9.0)
             chosen = VXB_VARIANT_DECODE_ROWS;
             char unused[8];
             // one or two fp32 rows: the single-launch form.  From three rows on every CTA repeating the
