@@ -309,13 +309,13 @@ __device__ __forceinline__ void gemm_i8_pair_body(const GemmTcgen05Args& args) {
                 s_ws[i] = wsv; s_bias[i] = bv;
             }
             __syncwarp();
+            const uint32_t row = m0 + quarter * 32 + lane;
+            const bool row_ok = row < args.rows;
+            const float as = (row_ok && ep.mode != kEpiAcc) ? epi_row_scale(ep, row) : 1.0f;   // (rows beyond the batch: any scale)
             ok = __all_sync(0xffffffffu, mbar_wait(sm.tmem_full(acc), acc_phase, abort_flag));
             if (!ok) break;
             tc_fence_after();
 
-            const uint32_t row = m0 + quarter * 32 + lane;
-            const bool row_ok = row < args.rows;
-            const float as = (row_ok && ep.mode != kEpiAcc) ? epi_row_scale(ep, row) : 1.0f;   // (rows beyond the batch: any scale)
             const bool fast = ep.fast_div != 0 && div_const_row_ok(as);
             const uint32_t taddr = tmem_base + ((quarter * 32u) << 16) + acc * kAccCols + cbase;
 #pragma unroll 1

@@ -208,14 +208,14 @@ gemm_i8_wide_kernel(const __grid_constant__ GemmTcgen05Args args) {
                 s_ws[i] = wsv; s_bias[i] = bv;
             }
             __syncwarp();
+            const uint32_t row = m0 + quarter * 32 + lane;
+            const bool row_ok = row < args.rows;
+            const float as = (row_ok && ep.mode == kEpiF32) ? __ldg(ep.row_scales + row) : 0.0f;
             ok = __all_sync(0xffffffffu, mbar_wait(sm.tmem_full(acc), acc_phase, abort_flag));
             if (!ok) break;
             tc_fence_after();
             if (t == blockIdx.x && ew == 0) stamp(args.trace, 4);
 
-            const uint32_t row = m0 + quarter * 32 + lane;
-            const bool row_ok = row < args.rows;
-            const float as = (row_ok && ep.mode == kEpiF32) ? __ldg(ep.row_scales + row) : 0.0f;
             const uint64_t as2 = f32x2(as, as);
             const uint32_t taddr = tmem_base + ((quarter * 32u) << 16) + acc * kAccCols + cbase;
 #pragma unroll 1
