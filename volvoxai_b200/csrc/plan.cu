@@ -218,15 +218,7 @@ int vxb_plan(const VxbPlanQuery* query, VxbLaunchPlan* out, char* why, uint32_t 
             // one or two fp32 rows: the single-launch form.  From three rows on every CTA repeating the
             // quantization costs more than the separate cluster quantizer (17.1 against 15.5 us per
             // step at 8 rows, K 4096, N 14336), so the two-launch form stays.
-            // Nor for two rows where a CTA's share of the weights is too small to hide it: padded K of 2048 and more, share
-            // under 96 KB (graph replay, one launch / two: 2560 -> 1256 9.2 / 8.1 us, 4096 -> 1024 10.8 / 9.7, 8192 -> 1024
-            // 17.3 / 13.5; with a share of 224 KB 8192 -> 4096 12.4 / 12.7).  A single row and shorter rows keep the one
-            // launch: most of what the GPU saves there the second launch costs the host.
-            uint32_t tile = 0, tiles_per_cta = 0;
-            decode_rows_plan(q.n, (int)sms, &tile, &tiles_per_cta);
-            const uint32_t kpad = round_up(q.k, kKAlign);
-            const bool hidden = q.rows == 1 || kpad < 2048u || (uint64_t)tile * tiles_per_cta * kpad >= 96u * 1024u;
-            if (q.fp32_input && q.rows <= tunables().decode_fused_max_rows && hidden &&
+            if (q.fp32_input && q.rows <= tunables().decode_fused_max_rows &&
                 admitted(kVariants[VXB_VARIANT_DECODE_FUSED], q, unused, sizeof unused)) chosen = VXB_VARIANT_DECODE_FUSED;
         }
         else {
