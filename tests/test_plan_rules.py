@@ -1,0 +1,39 @@
+"""Where the automatic routes change over (no GPU): each rule at its line and on both sides of it."""
+import pytest
+
+from volvoxai_b200 import _lib, w8a8
+
+
+def pick(rows, k, n, **kw):
+    plan, why = w8a8.plan(rows, k, n, sm_count=148, **kw)
+    assert plan is not None, why
+    return plan
+
+
+@pytest.mark.parametrize("rows,k,n,decode", [(64, 4096, 14336, True), (65, 1024, 3072, True), (128, 1024, 3073, False), (65, 1025, 64, False),
+                                             (128, 576, 64, True)])
+def test_rows_past_64_keep_the_decode_kernel_for_small_weights_only(rows, k, n, decode):
+    for epilogue in (_lib.EPI_ACC, _lib.EPI_F32, _lib.EPI_I8):
+        assert (pick(rows, k, n, epilogue=epilogue)["id"] == "DECODE_ROWS") == decode
+
+
+@pytest.mark.parametrize("rows,k,n,want", [(512, 4096, 4096, "TCGEN05_PAIR_NARROW"), (1024, 4096, 4096, "TCGEN05"), (2048, 4096, 4096, "TCGEN05_PAIR"),
+                                           (512, 1536, 4096, "TCGEN05"), (512, 1537, 4096, "TCGEN05_PAIR_NARROW")])
+def test_long_k_takes_the_cheapest_waves(rows, k, n, want):
+    assert pick(rows, k, n, epilogue=_lib.EPI_I8)["id"] == want
+    plan = pick(rows, k, n, epilogue=_lib.EPI_I8, pair_clusters=0)
+    assert plan["id"] == "TCGEN05"
+
+
+def test_silu_tail_from_a_full_wave_of_tiles():
+    assert pick(4096, 576, 3072, fused_tail=2)["id"] == "TCGEN05_WIDE_SILU"
+    assert pick(1280, 576, 3584, fused_tail=2)["id"] == "TCGEN05"                  # 140 tiles
+    assert pick(1408, 576, 3584, fused_tail=2)["id"] == "TCGEN05_WIDE_SILU"        # 154
+    assert pick(4096, 576, 3072, fused_tail=2, out_store_aligned=False)["id"] == "TCGEN05_PAIR"
+    assert pick(4096, 1537, 3072, fused_tail=2)["id"] == "TCGEN05_PAIR"
+
+
+@pytest.mark.parametrize("rows,n,tile", [(64, 14336, (64, 128)), (8, 14336, (16, 128)), (8, 9472, (16, 64)), (17, 9473, (32, 128)), (65, 4096, (128, 128))])
+def test_grouped_rows_up_to_64_have_the_weights_as_m(rows, n, tile):
+    plan = pick(rows, 4096, n, weight_kind=_lib.WEIGHT_GROUPED, group_size=128)
+    assert plan["id"] == "GROUPED_TCGEN05" and (plan["tile_rows"], plan["tile_columns"]) == tile

@@ -284,8 +284,11 @@ decode_rows_kernel(const __grid_constant__ DecodeRowsArgs args) {
     float* s_bias = s_ws + kMaxTile;
     int32_t* s_xpose = reinterpret_cast<int32_t*>(base + lay.xpose_off());
 
-    // let the next launch in the stream become resident as early as possible (see kPairSmemBytes)
-    if (threadIdx.x == 0) { pdl_release(); stamp(args.trace, 0); }
+    // Let the next launch in the stream become resident as early as possible (see kPairSmemBytes).  Not so in the
+    // single-launch form: there the next launch's set-up and first weights on the same SM held up this one's
+    // quantization, so it is let in when that is done (graph replay, one row 576 -> 1536 6.8 -> 6.1 us, 2560 -> 1256
+    // 8.7 -> 7.5, 8192 -> 1024 15.1 -> 13.2; two rows 2560 -> 1256 9.2 -> 8.0).
+    if (threadIdx.x == 0) { if (!args.x_f32) pdl_release(); stamp(args.trace, 0); }
 
     const uint32_t num_kb = args.kpad / kRK;
     const uint32_t tiles = args.tiles_per_cta;
@@ -351,6 +354,7 @@ decode_rows_kernel(const __grid_constant__ DecodeRowsArgs args) {
                                 ModeCfg<PAIR>::kThreads / 32, args.norm_weight, args.norm_eps, args.norm_out, part_ss);
             fence_proxy_async();   // generic-proxy writes to shared memory -> visible to the tensor core's reads
             __syncthreads();
+            if (threadIdx.x == 0) pdl_release();
         }
     }
 
