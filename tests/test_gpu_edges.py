@@ -192,8 +192,8 @@ def test_wide_silu_tiles(torch, ctx, rows, k, n):
 
 @pytest.mark.parametrize("rows,k", [(1, 64), (5, 1000), (64, 1024), (700, 576), (40, 9000)])
 def test_rmsnorm_products_near_and_far_from_one(torch, ctx, rows, k):
-    """The normalized rows against the same arithmetic in 64 bits: ordinary rows, rows scaled to 1e-25 and 1e25 (the
-    products leave the range of the split form), gammas of 0, 1e-33 and 1e30."""
+    """The normalized rows against the same arithmetic in 64 bits: ordinary rows, rows scaled to 1e-25 and 1e25, gammas
+    of 0, 1e-33 and 1e30."""
     rng = np.random.default_rng(rows + k)
     x = rng.standard_normal((rows, k)).astype(np.float32)
     x[rows // 2] *= np.float32(1e-25)
@@ -206,6 +206,36 @@ def test_rmsnorm_products_near_and_far_from_one(torch, ctx, rows, k):
     y = y.cpu().numpy()
     # one rounding to fp32 each; a 64-bit rounding can tip it in a handful of elements, by one place
     assert (np.abs(y.view(np.int32).astype(np.int64) - want.view(np.int32)) <= 1).all() and (y != want).mean() <= 1e-4
+
+
+@pytest.mark.parametrize("tiny,gain", [(1e-33, 1e15), (3e-36, 1e16), (1.35 * 2.0 ** -100, 1.77 * 2.0 ** 60), (1e-38, 1e18)])
+@pytest.mark.parametrize("form", ["aligned", "unaligned", "single launch"])
+def test_rmsnorm_tiny_elements_under_large_gammas(torch, ctx, form, tiny, gain):
+    """Elements whose normalized value x * inv lies near or below the smallest fp32 and comes back into range by a large
+    gamma, in rows with an rms of about 1e9: every form of the operator within one place of 64 bits."""
+    from volvoxai_b200 import w8a8
+    rows, k = 2, 640
+    rng = np.random.default_rng(5)
+    x = (rng.standard_normal((rows, k)) * 1e9).astype(np.float32)
+    g = (1 + 0.1 * rng.standard_normal(k)).astype(np.float32)
+    x[:, 7::64] = tiny * rng.uniform(0.5, 2, size=(rows, 10))
+    g[7::64] = gain * rng.uniform(0.5, 2, size=10)
+    x64 = x.astype(np.float64)
+    want = (x64 / np.sqrt((x64 ** 2).mean(axis=1, keepdims=True) + float(np.float32(1e-6))) * g.astype(np.float64)).astype(np.float32)
+    if form == "single launch":
+        c = wl.single_linear(rows=rows, k=k, n=64, seed=3)
+        weight = w8a8.Weight.from_i8(ctx, c["w"], c["ws"])
+        y = torch.empty((rows, k), device="cuda")
+        ctx.rmsnorm_linear_f32_fused(weight, dev(torch, x), dev(torch, g), 1e-6, norm_out=y)
+        assert "decode-fused" in w8a8.last_route()
+        weight.close()
+    else:
+        flat = torch.empty(rows * k + 1, device="cuda")
+        at = 1 if form == "unaligned" else 0
+        flat[at:at + rows * k] = dev(torch, x).flatten()
+        y = ctx.rmsnorm_quantize_rows(flat[at:at + rows * k].view(rows, k), dev(torch, g), 1e-6, ldq=k)[0]
+    y = y.cpu().numpy()
+    assert (np.abs(bits(y).astype(np.int64) - bits(want).astype(np.int64)) <= 1).all()
 
 
 @pytest.mark.parametrize("rows,k,n", [(65, 1024, 3080), (100, 1152, 200), (128, 4096, 1000), (66, 64, 4000)])

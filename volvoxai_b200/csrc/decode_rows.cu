@@ -203,7 +203,7 @@ __device__ __forceinline__ void fused_quantize_rows(const float* __restrict__ x,
         if (threadIdx.x < rows) {
             double t = 0.0;
             for (uint32_t i = 0; i < wpr; i++) t += part_ss[threadIdx.x * wpr + i];
-            part_ss[32 + threadIdx.x] = 1.0 / sqrt(t / (double)k + eps);
+            part_ss[32 + threadIdx.x] = row_inverse(t, k, eps);
         }
         __syncthreads();
         if (active) inv = part_ss[32 + row];

@@ -358,7 +358,7 @@ cudaError_t launch_any(const float* x, uint32_t rows, uint32_t k, int8_t* q, uin
 // stream once: normalize, (optionally) persist the normalized row for other consumers, quantize.
 // Arithmetic of the normalization follows the reference's CPU operator
 // (native/src/kernels/softmax_rmsnorm.inc:3-16): squares and their mean in double,
-// inv = 1 / sqrt(mean + eps) in double, y = float((double(x) * inv) * double(gamma)) (products: norm4).  The squares
+// inv = 1 / sqrt(mean + eps) in double, y = float((double(x) * inv) * double(gamma)).  The squares
 // are exact in double; only the order of the double additions differs from the sequential loop
 // (tree instead of left to right), which moves the mean by at most a few units of 2^-53.
 
@@ -399,7 +399,6 @@ rmsnorm_quantize_rows_vec(const float* __restrict__ x, const float* __restrict__
     const float4* in = reinterpret_cast<const float4*>(x + (size_t)(active ? row : 0) * k);
     const float4* g4 = reinterpret_cast<const float4*>(gamma);
     float4* nout = norm_out ? reinterpret_cast<float4*>(norm_out + (size_t)(active ? row : 0) * k) : nullptr;
-    const double inv_k = 1.0 / (double)k;   // long done when the sum is
 
     float4 cache[CACHE ? kMaxVecPerThread : 1];
     double ss = 0.0, ss2 = 0.0;
@@ -424,9 +423,9 @@ rmsnorm_quantize_rows_vec(const float* __restrict__ x, const float* __restrict__
     // one thread per row does the double-precision division and square root (slow, shared units); the others
     // take the result from shared memory
     __shared__ double smem_inv[kThreads / 8];
-    if (t == 0) smem_inv[threadIdx.x / THREADS_PER_ROW] = rsqrt(ss * inv_k + eps);
+    if (t == 0) smem_inv[threadIdx.x / THREADS_PER_ROW] = row_inverse(ss, k, eps);
     if constexpr (THREADS_PER_ROW > 32) __syncthreads(); else __syncwarp();
-    const RowInverse inv(smem_inv[threadIdx.x / THREADS_PER_ROW]);
+    const double inv = smem_inv[threadIdx.x / THREADS_PER_ROW];
 
     float amax = 0.0f; int bad = 0;
     if (active) {
@@ -493,7 +492,7 @@ rmsnorm_quantize_rows_scalar(const float* __restrict__ x, const float* __restric
     for (uint32_t j = lane; j < k; j += 32) ss = __fma_rn((double)in[j], (double)in[j], ss);
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
-    const double inv = rsqrt(ss / (double)k + eps);
+    const double inv = row_inverse(ss, k, eps);
     float amax = 0.0f; int bad = 0;
     for (uint32_t j = lane; j < k; j += 32) {
         const float v = norm1(in[j], inv, gamma[j]);

@@ -80,39 +80,19 @@ __device__ __forceinline__ float row_scale_from_amax(float amax) {
 
 // RMSNorm in front of the quantizer (the reference's CPU operator, native/src/kernels/softmax_rmsnorm.inc:3-16):
 // squares and their mean in double, inv = 1 / sqrt(mean + eps) in double, y = float((double(x) * inv) * double(gamma)).
+// Every form of the operator takes its inverse and its products from here: forms differ in the order of the double
+// additions alone, which moves the mean by a few units of 2^-53 and a normalized value by one place in about 2^-27 of
+// the elements.
+// The products stay in double: as fp32 pairs with their rounding errors carried along they held 48 bits of the 53 and
+// only while x * inv, not the result alone, kept away from the exponent limits, and bought less than a microsecond a
+// launch (pairs / double): 64 x 1024 2.7 / 2.7, 512 x 4096 5.9 / 6.1, 2048 x 2048 10.0 / 10.6, 4096 x 576 6.1 / 6.9,
+// 8192 x 4096 50.4 / 49.9 us; a layer of 4096 rows with two of them 79.9 / 80.9.
+__device__ __forceinline__ double row_inverse(double ss, uint32_t k, double eps) { return 1.0 / sqrt(ss / (double)k + eps); }
 __device__ __forceinline__ float norm1(float x, double inv, float g) {
     return __double2float_rn(__dmul_rn(__dmul_rn((double)x, inv), (double)g));
 }
 __device__ __forceinline__ float4 norm4(float4 c, double inv, float4 g) {
     return make_float4(norm1(c.x, inv, g.x), norm1(c.y, inv, g.y), norm1(c.z, inv, g.z), norm1(c.w, inv, g.w));
-}
-// The same with fp32 instructions where nothing comes near the exponent limits: inv = hi + lo to 2^-48, both products
-// with their rounding errors carried along (exact fused residuals), one rounding at the end - the fp32 nearest to
-// x * inv * g but for a relative 2^-46 around the ties, as from double.  Seven fp32 instructions instead of two
-// double products and three conversions, which run at an eighth of the rate and less.  With the wider rows of few-row
-// launches: 64 x 1024 5.0 -> 2.7 us, 512 x 4096 7.8 -> 5.3.
-struct RowInverse {
-    double inv;
-    float hi, lo;
-    bool split;    // false: only the double form is safe (a row of zeros, infinities, NaN, or far from 1)
-    __device__ __forceinline__ explicit RowInverse(double v) : inv(v) {
-        hi = __double2float_rn(v);
-        lo = __double2float_rn(v - (double)hi);
-        split = v >= 0x1p-60 && v <= 0x1p60;
-    }
-};
-__device__ __forceinline__ float norm1_split(float x, const RowInverse& r, float g, bool& far) {
-    const float p = __fmul_rn(x, r.hi);
-    const float e = __fmaf_rn(x, r.lo, __fmaf_rn(x, r.hi, -p));
-    const float y = __fmul_rn(p, g);
-    far |= !(fabsf(y) >= 0x1p-100f && fabsf(y) <= 0x1p100f);   // zeros, NaN, and products whose residual could underflow
-    return __fadd_rn(y, __fmaf_rn(e, g, __fmaf_rn(p, g, -y)));
-}
-__device__ __forceinline__ float4 norm4(float4 c, const RowInverse& r, float4 g) {
-    bool far = !r.split;
-    const float4 y = make_float4(norm1_split(c.x, r, g.x, far), norm1_split(c.y, r, g.y, far),
-                                 norm1_split(c.z, r, g.z, far), norm1_split(c.w, r, g.w, far));
-    return far ? norm4(c, r.inv, g) : y;
 }
 __device__ __forceinline__ double square_sum4(float4 c, double acc) {
     acc = __fma_rn((double)c.x, (double)c.x, acc);
