@@ -82,6 +82,31 @@ def test_word_outputs_on_any_boundary(torch, ctx, n, lead):
     weight.close()
 
 
+@pytest.mark.parametrize("n", [4, 28, 36, 64, 132, 260, 2052])
+@pytest.mark.parametrize("rows", [129, 150, 289])
+def test_word_outputs_on_eight_byte_boundaries(torch, ctx, rows, n):
+    """fp32 tiles and their SiLU * Mul form in a window whose rows start on 8 bytes and not on 16 (stored in pairs of
+    words), and on 4 (in words): equal to the 16-byte aligned form, nothing written beside the window."""
+    from volvoxai_b200 import w8a8
+    c = wl.single_linear(rows=rows, k=100, n=n, seed=n + rows)
+    weight = w8a8.Weight.from_i8(ctx, c["w"], c["ws"], bias_f32=c["bias"])
+    x = dev(torch, c["x"])
+
+    def window(width, lead, pitch, call):
+        wide = torch.full((rows, pitch), 99.0, device="cuda")
+        call(wide[:, lead:lead + width])
+        assert (wide[:, :lead] == 99).all() and (wide[:, lead + width:] == 99).all()
+        return wide[:, lead:lead + width].clone()
+
+    calls = [(n, lambda out, r=r: ctx.linear_f32(weight, x, out=out, route=r)) for r in (w8a8.ROUTE_TCGEN05, w8a8.ROUTE_TCGEN05_PAIR)]
+    calls.append((n // 2, lambda out: ctx.linear_f32_fused(weight, x, silu_mul=True, out=out)))
+    for width, call in calls:
+        want = window(width, 0, (width + 7) // 4 * 4, call)
+        for lead, pitch in ((2, width + 2 + width % 2), (2, width + 4 + width % 2), (1, width + 1), (2, width + 3 - width % 2)):
+            assert torch.equal(window(width, lead, pitch, call), want)
+    weight.close()
+
+
 @pytest.mark.parametrize("rows,k,n", [(129, 1600, 128), (257, 2048, 100), (512, 2000, 4096), (600, 4096, 1000), (300, 1537, 386)])
 def test_narrow_pair_tiles(torch, ctx, rows, k, n):
     """Long K and few tiles: 256 x 128 tiles by pairs of CTAs, every kind of output, equal to the single-CTA kernel."""

@@ -59,9 +59,39 @@ static __device__ __noinline__ void flush_bytes(const uint8_t* tile, uint32_t la
 
 // ---- 32-bit words: a [16 rows x 128 B] tile ------------------------------------------------------
 
+// 16 rows of the tile to out (row pitch ld words, rows [0, rows), columns [0, columns)) in pairs of words (two rows per
+// instruction) where base, pitch and width allow, else in words (a row per instruction).  All reads go ahead of the
+// stores: 4096 x 576 -> 2050, quantizer included, takes 19.3 us; read and stored one after the other, with a test of the
+// row between, it took 28.8, and in 16-byte pieces of four rows, split where not aligned, 20.8.  Not inlined, like flush_bytes.
+static __device__ __noinline__ void flush_words(const uint8_t* tile, uint32_t lane, uint32_t* out, uint32_t ld, uint32_t rows, uint32_t columns) {
+    if (((((uint32_t)(uintptr_t)out >> 2) | ld | columns) & 1u) == 0) {
+        const uint32_t l = lane & 15u, odd = lane >> 4;
+        const bool live = 2u * l < columns;
+        uint32_t* dst = out + (size_t)odd * ld + 2u * l;
+        uint2 v[8];
+#pragma unroll
+        for (uint32_t i = 0; i < 8; i++) {
+            const uint32_t r = 2u * i + odd;
+            v[i] = *reinterpret_cast<const uint2*>(tile + r * 128u + (((l >> 1) ^ (r & 7u)) << 4) + (l & 1u) * 8u);
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < 8; i++, dst += 2u * (size_t)ld)
+            if (live && 2u * i + odd < rows) *reinterpret_cast<uint2*>(dst) = v[i];
+    } else {
+        const bool live = lane < columns;
+        uint32_t* dst = out + lane;
+        uint32_t v[16];
+#pragma unroll
+        for (uint32_t i = 0; i < 16; i++) v[i] = *reinterpret_cast<const uint32_t*>(tile + i * 128u + (((lane >> 2) ^ (i & 7u)) << 4) + (lane & 3u) * 4u);
+#pragma unroll
+        for (uint32_t i = 0; i < 16; i++, dst += ld)
+            if (live && i < rows) *dst = v[i];
+    }
+}
+
 // One 32 x 32 chunk, this lane's row in o, to out (row pitch ld words, rows [0, rows), columns [0, columns)).
 // `aligned` (uniform): all 32 columns exist and every row segment is 16-byte aligned - four rows of 128 bytes per
-// instruction; otherwise a row per instruction, a word per lane.
+// instruction; otherwise flush_words.
 __device__ __forceinline__ void store_words(uint8_t* tile, uint32_t lane, const uint32_t (&o)[32], uint32_t* out, uint32_t ld,
                                             uint32_t rows, uint32_t columns, bool aligned) {
 #pragma unroll
@@ -83,17 +113,41 @@ __device__ __forceinline__ void store_words(uint8_t* tile, uint32_t lane, const 
                 if (half * 16u + r < rows) *reinterpret_cast<uint4*>(out + (size_t)(half * 16u + r) * ld + 4u * piece) = v;
             }
         } else {
-#pragma unroll 4
-            for (uint32_t r = 0; r < 16; r++) {
-                if (half * 16u + r >= rows) break;
-                const uint32_t v = *reinterpret_cast<const uint32_t*>(tile + r * 128u + (((lane >> 2) ^ (r & 7u)) << 4) + (lane & 3u) * 4u);
-                if (lane < columns) out[(size_t)(half * 16u + r) * ld + lane] = v;
-            }
+            const uint32_t r0 = half * 16u;
+            flush_words(tile, lane, out + (size_t)r0 * ld, ld, rows > r0 ? rows - r0 : 0u, columns);
         }
     }
 }
 
 // ---- 32-bit words, half as many columns: a [32 rows x 64 B] tile ----------------------------------
+
+// The same for a tile of half rows, all 32 of them: four rows per instruction in pairs of words, two in words.
+static __device__ __noinline__ void flush_half_words(const uint8_t* tile, uint32_t lane, float* out, uint32_t ld, uint32_t rows, uint32_t columns) {
+    if (((((uint32_t)(uintptr_t)out >> 2) | ld | columns) & 1u) == 0) {
+        const uint32_t l = lane & 7u, sub = lane >> 3;
+        const bool live = 2u * l < columns;
+        float* dst = out + (size_t)sub * ld + 2u * l;
+        float2 v[8];
+#pragma unroll
+        for (uint32_t i = 0; i < 8; i++) {
+            const uint32_t r = 4u * i + sub;
+            v[i] = *reinterpret_cast<const float2*>(tile + r * 64u + (((l >> 1) ^ ((r >> 1) & 3u)) << 4) + (l & 1u) * 8u);
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < 8; i++, dst += 4u * (size_t)ld)
+            if (live && 4u * i + sub < rows) *reinterpret_cast<float2*>(dst) = v[i];
+    } else {
+        const uint32_t l = lane & 15u, odd = lane >> 4;
+        const bool live = l < columns;
+        float* dst = out + (size_t)odd * ld + l;
+        float v[16];
+#pragma unroll
+        for (uint32_t i = 0; i < 16; i++) v[i] = *reinterpret_cast<const float*>(tile + (2u * i + odd) * 64u + (((l >> 2) ^ (i & 3u)) << 4) + (l & 3u) * 4u);
+#pragma unroll
+        for (uint32_t i = 0; i < 16; i++, dst += 2u * (size_t)ld)
+            if (live && 2u * i + odd < rows) *dst = v[i];
+    }
+}
 
 // The SiLU * Mul tail leaves 16 outputs of a 32-channel chunk: this lane's row in y, to out as store_words does.
 __device__ __forceinline__ void store_half_words(uint8_t* tile, uint32_t lane, const float (&y)[16], float* out, uint32_t ld,
@@ -112,12 +166,7 @@ __device__ __forceinline__ void store_half_words(uint8_t* tile, uint32_t lane, c
             if (r < rows) *reinterpret_cast<float4*>(out + (size_t)r * ld + 4u * piece) = v;
         }
     } else {
-        const uint32_t l = lane & 15u;
-#pragma unroll 4
-        for (uint32_t r = lane >> 4; r < 32u; r += 2u) {
-            if (r >= rows) break;
-            if (l < columns) out[(size_t)r * ld + l] = *reinterpret_cast<const float*>(tile + r * 64u + (((l >> 2) ^ ((r >> 1) & 3u)) << 4) + (l & 3u) * 4u);
-        }
+        flush_half_words(tile, lane, out, ld, rows, columns);
     }
 }
 
