@@ -38,6 +38,23 @@ def test_quantizer_any_width_and_alignment(torch, ctx, oracle, k, rows):
     assert np.array_equal(bits(s[vo != 0]), bits(so[vo != 0])) and np.isnan(s[vo == 0]).all()
 
 
+@pytest.mark.parametrize("rows,k", [(r, k + d) for r, ks in ((5000, (128, 256, 512, 1024)), (3, (256, 512, 1024, 2048, 4096, 8192))) for k in ks for d in (0, 1)])
+def test_quantizer_elements_per_thread(torch, ctx, oracle, rows, k):
+    """Widths on both sides of each step in the any-alignment quantizer's elements per thread, with 32 threads per row and
+    with up to 256."""
+    x = np.random.default_rng(k + rows).standard_normal((rows, k)).astype(np.float32)
+    x[1, k - 1] = -np.inf
+    x[2] *= np.float32(1e-36)
+    qo, so, vo = oracle.quantize_rows(x)
+    flat = torch.empty(rows * k + 1, device="cuda")
+    flat[1:] = dev(torch, x).flatten()
+    kpad = (k + 127) // 128 * 128
+    q, s, v = (t.cpu().numpy() for t in ctx.quantize_rows(flat[1:].view(rows, k), ldq=kpad))
+    assert np.array_equal(v != 0, vo != 0)
+    assert np.array_equal(q[:, :k], qo) and (q[:, k:] == 0).all()
+    assert np.array_equal(bits(s[vo != 0]), bits(so[vo != 0])) and np.isnan(s[vo == 0]).all()
+
+
 @pytest.mark.parametrize("n", [1, 3, 31, 33, 62, 64, 66, 97, 129, 250, 257, 514])
 @pytest.mark.parametrize("rows,lead,extra", [(129, 0, 0), (161, 1, 2), (300, 2, 5), (140, 16, 32), (131, 4, 8)])
 def test_byte_outputs_on_any_boundary(torch, ctx, n, rows, lead, extra):

@@ -205,11 +205,12 @@ cudaError_t launch_cluster(const float* x, uint32_t rows, uint32_t k, int8_t* q,
 
 // Any k, any alignment: thread t of a row's THREADS_PER_ROW takes the elements t, t + THREADS_PER_ROW, ..., so
 // that every load instruction covers 128 consecutive bytes per warp and every (byte) store a whole sector of the
-// padded code row, whatever the row's first byte is.  CACHE: up to 32 elements per thread stay in registers
-// between the absmax and the quantizing pass (K <= 8192).  Alone, 4096 x 4099: 24.2 us (3.5 TB/s), 777 x 1283: 5.7;
-// one warp per row, reading the row twice in steps of 32 elements, took 64.8 and 6.2.
+// padded code row, whatever the row's first byte is.  PER: at most so many elements per thread, which stay in registers
+// between the absmax and the quantizing pass; 0: rows of more than 8192 elements, read twice.  Alone, one warp per row that
+// reads it twice / 32 elements per thread for every width, which a narrow row paid for / the width's own number: 4096 x
+// 4099 64.8 / 24.7 / 24.7 us, 777 x 1283 6.3 / 5.7 / 3.4, 2048 x 576 6.1 / 7.1 / 3.5, 4096 x 128 3.3 / 5.2 / 1.9.
 constexpr int kMaxPerThread = 4 * kMaxVecPerThread;
-template <int THREADS_PER_ROW, bool CACHE>
+template <int THREADS_PER_ROW, int PER>
 __global__ void __launch_bounds__(kThreads)
 quantize_rows_any(const float* __restrict__ x, uint32_t rows, uint32_t k, int8_t* __restrict__ q,
                   uint32_t ldq, float* __restrict__ row_scales, int32_t* __restrict__ valid) {
@@ -223,17 +224,17 @@ quantize_rows_any(const float* __restrict__ x, uint32_t rows, uint32_t k, int8_t
     const bool active = row < rows;
     const float* in = x + (size_t)(active ? row : 0) * k;
 
-    float cache[CACHE ? kMaxPerThread : 1];
+    float cache[PER ? PER : 1];
     float amax = 0.0f; int bad = 0;
     if (active) {
-        if constexpr (CACHE) {
+        if constexpr (PER != 0) {
 #pragma unroll
-            for (int i = 0; i < kMaxPerThread; i++) {
+            for (int i = 0; i < PER; i++) {
                 const uint32_t j = t + i * THREADS_PER_ROW;
                 cache[i] = j < k ? __ldg(in + j) : 0.0f;
             }
 #pragma unroll
-            for (int i = 0; i < kMaxPerThread; i++) {
+            for (int i = 0; i < PER; i++) {
                 bad |= nonfinite_bits(cache[i]);
                 amax = fmaxf(amax, fabsf(cache[i]));
             }
@@ -257,11 +258,11 @@ quantize_rows_any(const float* __restrict__ x, uint32_t rows, uint32_t k, int8_t
     int8_t* out = q + (size_t)row * ldq;
     const RowDivisor div(scale);
     uint32_t done = 0;
-    if constexpr (CACHE) {
+    if constexpr (PER != 0) {
         if (div.fast && !bad) {
             const uint64_t rcp2 = f32x2(div.rcp, div.rcp), neg_d2 = f32x2(-div.scale, -div.scale);
 #pragma unroll
-            for (int i = 0; i < kMaxPerThread; i += 2) {
+            for (int i = 0; i < PER; i += 2) {
                 const uint32_t j = t + i * THREADS_PER_ROW;
                 int32_t a, b;
                 quant2_fast(cache[i], cache[i + 1], rcp2, neg_d2, a, b);   // zero past the row's end: code 0
@@ -270,12 +271,12 @@ quantize_rows_any(const float* __restrict__ x, uint32_t rows, uint32_t k, int8_t
             }
         } else {
 #pragma unroll
-            for (int i = 0; i < kMaxPerThread; i++) {
+            for (int i = 0; i < PER; i++) {
                 const uint32_t j = t + i * THREADS_PER_ROW;
                 if (j < ldq) out[j] = (j < k && !bad) ? (int8_t)quant1<false>(cache[i], div) : (int8_t)0;
             }
         }
-        done = kMaxPerThread * THREADS_PER_ROW;
+        done = PER * THREADS_PER_ROW;
     }
 #pragma unroll 8
     for (uint32_t j = done + t; j < ldq; j += THREADS_PER_ROW)
@@ -342,14 +343,21 @@ cudaError_t launch_vec(const float* x, uint32_t rows, uint32_t k, int8_t* q, uin
                       x, rows, k, q, ldq, row_scales, valid);
 }
 
+template <int TPR, int PER>
+cudaError_t launch_any_per(const float* x, uint32_t rows, uint32_t k, int8_t* q, uint32_t ldq,
+                           float* row_scales, int32_t* valid, cudaStream_t stream) {
+    constexpr uint32_t kRowsPerCta = kThreads / TPR;
+    return launch_pdl(quantize_rows_any<TPR, PER>, dim3((rows + kRowsPerCta - 1) / kRowsPerCta), dim3(kThreads), 0, stream,
+                      x, rows, k, q, ldq, row_scales, valid);
+}
 template <int TPR>
 cudaError_t launch_any(const float* x, uint32_t rows, uint32_t k, int8_t* q, uint32_t ldq,
                        float* row_scales, int32_t* valid, cudaStream_t stream) {
-    constexpr uint32_t kRowsPerCta = kThreads / TPR;
-    const uint32_t grid = (rows + kRowsPerCta - 1) / kRowsPerCta;
-    if (k <= (uint32_t)TPR * kMaxPerThread)
-        return launch_pdl(quantize_rows_any<TPR, true>, dim3(grid), dim3(kThreads), 0, stream, x, rows, k, q, ldq, row_scales, valid);
-    return launch_pdl(quantize_rows_any<TPR, false>, dim3(grid), dim3(kThreads), 0, stream, x, rows, k, q, ldq, row_scales, valid);
+    if (k <= (uint32_t)TPR * 4) return launch_any_per<TPR, 4>(x, rows, k, q, ldq, row_scales, valid, stream);
+    if (k <= (uint32_t)TPR * 8) return launch_any_per<TPR, 8>(x, rows, k, q, ldq, row_scales, valid, stream);
+    if (k <= (uint32_t)TPR * 16) return launch_any_per<TPR, 16>(x, rows, k, q, ldq, row_scales, valid, stream);
+    if (k <= (uint32_t)TPR * kMaxPerThread) return launch_any_per<TPR, kMaxPerThread>(x, rows, k, q, ldq, row_scales, valid, stream);
+    return launch_any_per<kThreads, 0>(x, rows, k, q, ldq, row_scales, valid, stream);   // (TPR is kThreads then)
 }
 
 
