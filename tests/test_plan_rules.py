@@ -37,3 +37,12 @@ def test_silu_tail_from_a_full_wave_of_tiles():
 def test_grouped_rows_up_to_64_have_the_weights_as_m(rows, n, tile):
     plan = pick(rows, 4096, n, weight_kind=_lib.WEIGHT_GROUPED, group_size=128)
     assert plan["id"] == "GROUPED_TCGEN05" and (plan["tile_rows"], plan["tile_columns"]) == tile
+
+
+@pytest.mark.parametrize("rows,k,per_row", [(64, 1024, 256), (128, 1024, 256), (148, 1024, 256), (149, 1024, 128), (296, 1024, 128), (297, 1024, 64), (592, 1024, 64),
+                                            (593, 1024, 32), (777, 576, 32), (300, 576, 64), (1184, 256, 32), (1185, 256, 8), (64, 124, 8), (64, 128, 32),
+                                            (148, 4096, 256), (149, 4096, 128), (8192, 4096, 128), (40, 8192, 256)])
+def test_quantizer_threads_per_row(rows, k, per_row):
+    """Doubled while the launch stays within 256 threads per SM and a thread keeps a float4."""
+    plan = pick(rows, k, 4096, fp32_input=True)
+    assert plan["quantizer"] == 2 and plan["quantizer_grid"] == -(-rows // (256 // per_row))

@@ -300,7 +300,7 @@ cudaError_t launch_rmsnorm_quantize_rows(const float* x, const float* gamma, flo
 cudaError_t launch_quantize_rows(const float* x, uint32_t rows, uint32_t k, int8_t* q,
                                  uint32_t ldq, float* row_scales, int32_t* valid,
                                  cudaStream_t stream);
-uint32_t quantize_vec_threads(uint32_t rows, uint32_t k);   // threads per row of the quantizers with 128-bit loads
+uint32_t quantize_vec_threads(uint32_t rows, uint32_t k, bool norm = false);   // threads per row of the quantizers with 128-bit loads
 uint32_t quantize_any_threads(uint32_t rows, uint32_t k);   // threads per row of the quantizer that takes any width and alignment
 
 // Activation bytes into the padded row layout, with U8 codes converted to the signed domain (x ^ 0x80).

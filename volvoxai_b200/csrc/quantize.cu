@@ -549,12 +549,19 @@ uint32_t quantize_any_threads(uint32_t rows, uint32_t k) {
     return tpr;
 }
 
-// ... with 128-bit loads: at most 8 float4 per thread, widened below a quarter of the chip's threads while every
-// thread keeps one (64 x 1024: 2.07 -> 1.76 us; 4096 x 576 would go from 3.3 to 4.5).
-uint32_t quantize_vec_threads(uint32_t rows, uint32_t k) {
+// ... with 128-bit loads: at most 8 float4 per thread, then doubled (from 8 to 32) while the whole launch stays within 256
+// threads per SM, 512 with the RMSNorm's longer row, and every thread keeps a float4.  More threads than that cost more in
+// row reductions and blocks than the loads in flight give, alone (us, never doubled / doubled from below 512 per SM to
+// below 1024 / this rule): 64 x 1024 2.1 / 1.8 / 1.8, 512 x 1024 2.2 / 2.8 / 2.1, 777 x 576 2.1 / 2.9 / 2.1, 2048 x 256
+// 2.2 / 2.8 / 2.1; with the norm 64 x 1024 4.9 / 2.7 / 2.7, 512 x 1024 5.2 / 4.2 / 3.3.
+uint32_t quantize_vec_threads(uint32_t rows, uint32_t k, bool norm) {
+    const uint64_t most = 148u * (norm ? 512u : 256u);
     uint32_t tpr = k <= 256 ? 8 : k <= 1024 ? 32 : k <= 2048 ? 64 : k <= 4096 ? 128 : 256;
-    while (tpr < (uint32_t)kThreads && (uint64_t)rows * tpr < 148u * 512u && k / 4u >= (tpr == 8 ? 32u : 2u * tpr)) tpr = tpr == 8 ? 32u : 2u * tpr;
-    return tpr;
+    for (;;) {
+        const uint32_t next = tpr == 8 ? 32u : 2u * tpr;
+        if (next > (uint32_t)kThreads || (uint64_t)rows * next > most || k / 4u < next) return tpr;
+        tpr = next;
+    }
 }
 
 cudaError_t launch_quantize_rows(const float* x, uint32_t rows, uint32_t k, int8_t* q, uint32_t ldq,
@@ -597,7 +604,7 @@ cudaError_t launch_rmsnorm_quantize_rows(const float* x, const float* gamma, flo
         return launch_pdl(rmsnorm_quantize_rows_scalar, dim3(grid), dim3(kThreads), 0, stream,
                           x, gamma, eps, rows, k, norm_out, q, ldq, row_scales, valid);
     }
-    switch (quantize_vec_threads(rows, k)) {
+    switch (quantize_vec_threads(rows, k, true)) {
         case 8: return launch_norm_vec<8>(x, gamma, eps, rows, k, norm_out, q, ldq, row_scales, valid, stream);
         case 32: return launch_norm_vec<32>(x, gamma, eps, rows, k, norm_out, q, ldq, row_scales, valid, stream);
         case 64: return launch_norm_vec<64>(x, gamma, eps, rows, k, norm_out, q, ldq, row_scales, valid, stream);
