@@ -295,3 +295,47 @@ def test_rows_past_64_in_tiles(torch, ctx, rows, k, n):
         assert torch.equal(y, call(w8a8.ROUTE_DECODE))
     assert torch.equal(ctx.linear_f32_fused(weight, x, residual=res), ctx.linear_f32(weight, x, route=w8a8.ROUTE_DECODE) + res)
     weight.close()
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_small_calls_back_to_back(torch, ctx, captured):
+    """Calls on both sides of the line up to which the quantizer lets its GEMM in before its own wait, and single-launch
+    calls on both sides of theirs, one after the other through one context's scratch without a pause, in a stream and
+    replayed from a graph: each output as when it is computed alone."""
+    from volvoxai_b200 import w8a8
+    shapes = [(6, 640, 1472), (8, 128, 300), (64, 1024, 1000), (16, 1024, 1000), (1, 576, 128), (3, 257, 64), (1, 576, 300), (33, 576, 200),
+              (128, 128, 600), (2, 1024, 64), (7, 2048, 500)]
+    weights, xs, want, outs = [], [], [], []
+    for i, (rows, k, n) in enumerate(shapes):
+        c = wl.single_linear(rows=rows, k=k, n=n, seed=i)
+        weights.append(w8a8.Weight.from_i8(ctx, c["w"], c["ws"], bias_f32=c["bias"]))
+        xs.append(dev(torch, c["x"]))
+        want.append(ctx.linear_f32(weights[i], xs[i], route=w8a8.ROUTE_SIMT))
+        outs.append(torch.empty_like(want[i]))
+        torch.cuda.synchronize()
+
+    def all_calls():
+        for w, x, y in zip(weights, xs, outs):
+            ctx.linear_f32(w, x, out=y)
+
+    stream = torch.cuda.Stream()
+    ctx.set_stream(stream.cuda_stream)
+    try:
+        with torch.cuda.stream(stream):
+            all_calls()
+            stream.synchronize()
+            graph = torch.cuda.CUDAGraph()
+            if captured:
+                with torch.cuda.graph(graph, stream=stream):
+                    all_calls()
+            for _ in range(20):
+                for y in outs:
+                    y.zero_()
+                graph.replay() if captured else all_calls()
+                stream.synchronize()
+                for y, ref in zip(outs, want):
+                    assert torch.equal(y, ref)
+    finally:
+        ctx.set_stream(None)
+    for w in weights:
+        w.close()

@@ -299,7 +299,7 @@ cudaError_t launch_rmsnorm_quantize_rows(const float* x, const float* gamma, flo
                                          float* row_scales, int32_t* valid, cudaStream_t stream);
 cudaError_t launch_quantize_rows(const float* x, uint32_t rows, uint32_t k, int8_t* q,
                                  uint32_t ldq, float* row_scales, int32_t* valid,
-                                 cudaStream_t stream);
+                                 cudaStream_t stream, bool early = false);   // early: the next launch is let in before the wait
 uint32_t quantize_vec_threads(uint32_t rows, uint32_t k, bool norm = false);   // threads per row of the quantizers with 128-bit loads
 uint32_t quantize_any_threads(uint32_t rows, uint32_t k);   // threads per row of the quantizer that takes any width and alignment
 

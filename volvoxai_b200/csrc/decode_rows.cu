@@ -79,6 +79,7 @@ template <uint32_t MT> struct RowsCfg {
 };
 
 constexpr uint32_t kMaxXSlots = 8;
+constexpr uint32_t kFewCtas = 18;           // an eighth of the SMs
 constexpr uint32_t kFusedMaxKpad = 8192;   // single-launch form: 8 rows x padded K of int8 stay in shared memory (64 KB at most)
 
 struct RowsLayout {       // dynamic shared memory, offsets from a 1024-byte aligned base
@@ -287,8 +288,11 @@ decode_rows_kernel(const __grid_constant__ DecodeRowsArgs args) {
     // Let the next launch in the stream become resident as early as possible (see kPairSmemBytes).  Not so in the
     // single-launch form: there the next launch's set-up and first weights on the same SM held up this one's
     // quantization, so it is let in when that is done (graph replay, one row 576 -> 1536 6.8 -> 6.1 us, 2560 -> 1256
-    // 8.7 -> 7.5, 8192 -> 1024 15.1 -> 13.2; two rows 2560 -> 1256 9.2 -> 8.0).
-    if (threadIdx.x == 0) { if (!args.x_f32) pdl_release(); stamp(args.trace, 0); }
+    // 8.7 -> 7.5, 8192 -> 1024 15.1 -> 13.2; two rows 2560 -> 1256 9.2 -> 8.0), unless this launch takes up so few SMs
+    // that the next one finds others (one row 576 -> 64 5.6 us let in at once, 5.8 after the quantization; 128 -> 64 5.1
+    // and 5.4; 576 -> 300, on 38 SMs, 5.7 and 6.0, but 6.7 and 6.2 in a stream of calls).  Once: a second signal costs
+    // the small launches 0.3 us.
+    if (threadIdx.x == 0) { if (!args.x_f32 || gridDim.x <= kFewCtas) pdl_release(); stamp(args.trace, 0); }
 
     const uint32_t num_kb = args.kpad / kRK;
     const uint32_t tiles = args.tiles_per_cta;
@@ -354,7 +358,7 @@ decode_rows_kernel(const __grid_constant__ DecodeRowsArgs args) {
                                 ModeCfg<PAIR>::kThreads / 32, args.norm_weight, args.norm_eps, args.norm_out, part_ss);
             fence_proxy_async();   // generic-proxy writes to shared memory -> visible to the tensor core's reads
             __syncthreads();
-            if (threadIdx.x == 0) pdl_release();
+            if (threadIdx.x == 0 && gridDim.x > kFewCtas) pdl_release();
         }
     }
 

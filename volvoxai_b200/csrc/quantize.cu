@@ -44,22 +44,29 @@ __device__ __forceinline__ void row_reduce(float& amax, int& bad, float* smem_ma
     }
 }
 
+// Every quantizer waits until the kernel before it has finished with the activations and the q scratch, and lets the
+// consumer kernel start its prologue and its first weight loads: after that wait as a rule, before it (`early`) where the
+// caller says so (api.cu's release_early).  Released before the wait, the consumer sets up and loads beside the
+// predecessor's last tiles and holds them up; released after it, its set-up is on the call's path.  us a pass, early /
+// late: 8 x 4096 -> 14336 in a stream of calls 16.7 / 15.8, replayed from a graph 15.9 / 15.4; 64 x 1024 -> 3072 8.3 / 7.2
+// and 7.6 / 6.8; decode layers replayed from a graph, 64 rows of hidden 1024 36.7 / 36.0, 8 rows of 576 28.4 / 25.8, 16 of
+// 2048 44.5 / 42.9 (41.4 / 38.3, 31.7 / 28.5, 47.4 / 45.2 in a stream).
+__device__ __forceinline__ void wait_and_release(bool early) {
+    if (early) pdl_release();
+    pdl_wait();
+    if (!early) pdl_release();
+}
+
 // THREADS_PER_ROW threads cooperate on one row; kThreads/THREADS_PER_ROW rows per CTA.
 // VEC: row addressed as float4 (k % 4 == 0, 16-byte aligned base and ldq % 16 == 0).
 // CACHE: the row's float4s stay in registers between the two passes.
 template <int THREADS_PER_ROW, bool CACHE>
 __global__ void __launch_bounds__(kThreads)
 quantize_rows_vec(const float* __restrict__ x, uint32_t rows, uint32_t k, int8_t* __restrict__ q,
-                  uint32_t ldq, float* __restrict__ row_scales, int32_t* __restrict__ valid) {
+                  uint32_t ldq, float* __restrict__ row_scales, int32_t* __restrict__ valid, bool early) {
     __shared__ float smem_max[kThreads / 32];
     __shared__ int smem_bad[kThreads / 32];
-    // Wait until the kernel before this one has finished with the activations and the q scratch; then let the consumer
-    // kernel start its prologue and weight prefetch (so in every quantizer).  Released before the wait, the consumer
-    // set up and loaded beside the predecessor's last tiles and held them up: one pass of a stream of calls, 8 x 4096 ->
-    // 14336 16.8 -> 15.9 us, 16 x 2048 -> 4096 9.3 -> 8.3, a decode layer of 64 rows 40.9 -> 38.2 (replayed from a graph
-    // 15.7 / 15.5, 8.4 / 8.6, 37.4 / 36.0; 6 x 640 -> 1472 5.9 / 6.4, 7.8 / 7.7 in a stream).
-    pdl_wait();
-    pdl_release();
+    wait_and_release(early);
     constexpr int kRowsPerCta = kThreads / THREADS_PER_ROW;
     const uint32_t row = blockIdx.x * kRowsPerCta + threadIdx.x / THREADS_PER_ROW;
     const int t = threadIdx.x % THREADS_PER_ROW;
@@ -132,14 +139,13 @@ quantize_rows_vec(const float* __restrict__ x, uint32_t rows, uint32_t k, int8_t
 template <int S>
 __global__ void __launch_bounds__(kThreads)
 quantize_rows_cluster(const float* __restrict__ x, uint32_t rows, uint32_t k, int8_t* __restrict__ q,
-                      uint32_t ldq, float* __restrict__ row_scales, int32_t* __restrict__ valid) {
+                      uint32_t ldq, float* __restrict__ row_scales, int32_t* __restrict__ valid, bool early) {
     namespace cg = cooperative_groups;
     __shared__ float smem_max[kThreads / 32];
     __shared__ int smem_bad[kThreads / 32];
     __shared__ float peer_max[S];
     __shared__ int peer_bad[S];
-    pdl_wait();
-    pdl_release();
+    wait_and_release(early);
     cg::cluster_group cluster = cg::this_cluster();
     const uint32_t rank = cluster.block_rank();
     const uint32_t row = blockIdx.y;
@@ -191,7 +197,7 @@ quantize_rows_cluster(const float* __restrict__ x, uint32_t rows, uint32_t k, in
 
 template <int S>
 cudaError_t launch_cluster(const float* x, uint32_t rows, uint32_t k, int8_t* q, uint32_t ldq,
-                           float* row_scales, int32_t* valid, cudaStream_t stream) {
+                           float* row_scales, int32_t* valid, cudaStream_t stream, bool early) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(S, rows); cfg.blockDim = dim3(kThreads); cfg.dynamicSmemBytes = 0; cfg.stream = stream;
     cudaLaunchAttribute attr[2];
@@ -200,7 +206,7 @@ cudaError_t launch_cluster(const float* x, uint32_t rows, uint32_t k, int8_t* q,
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr; cfg.numAttrs = 2;
-    return cudaLaunchKernelEx(&cfg, quantize_rows_cluster<S>, x, rows, k, q, ldq, row_scales, valid);
+    return cudaLaunchKernelEx(&cfg, quantize_rows_cluster<S>, x, rows, k, q, ldq, row_scales, valid, early);
 }
 
 // Any k, any alignment: thread t of a row's THREADS_PER_ROW takes the elements t, t + THREADS_PER_ROW, ..., so
@@ -213,11 +219,10 @@ constexpr int kMaxPerThread = 4 * kMaxVecPerThread;
 template <int THREADS_PER_ROW, int PER>
 __global__ void __launch_bounds__(kThreads)
 quantize_rows_any(const float* __restrict__ x, uint32_t rows, uint32_t k, int8_t* __restrict__ q,
-                  uint32_t ldq, float* __restrict__ row_scales, int32_t* __restrict__ valid) {
+                  uint32_t ldq, float* __restrict__ row_scales, int32_t* __restrict__ valid, bool early) {
     __shared__ float smem_max[kThreads / 32];
     __shared__ int smem_bad[kThreads / 32];
-    pdl_wait();
-    pdl_release();
+    wait_and_release(early);
     constexpr uint32_t kRowsPerCta = kThreads / THREADS_PER_ROW;
     const uint32_t row = blockIdx.x * kRowsPerCta + threadIdx.x / THREADS_PER_ROW;
     const uint32_t t = threadIdx.x % THREADS_PER_ROW;
@@ -333,31 +338,31 @@ repack_weight_kernel(const uint8_t* __restrict__ src, uint32_t src_ld, uint32_t 
 
 template <int TPR>
 cudaError_t launch_vec(const float* x, uint32_t rows, uint32_t k, int8_t* q, uint32_t ldq,
-                       float* row_scales, int32_t* valid, cudaStream_t stream) {
+                       float* row_scales, int32_t* valid, cudaStream_t stream, bool early) {
     constexpr int kRowsPerCta = kThreads / TPR;
     const uint32_t grid = (rows + kRowsPerCta - 1) / kRowsPerCta;
     if (k / 4 <= (uint32_t)TPR * kMaxVecPerThread)
         return launch_pdl(quantize_rows_vec<TPR, true>, dim3(grid), dim3(kThreads), 0, stream,
-                          x, rows, k, q, ldq, row_scales, valid);
+                          x, rows, k, q, ldq, row_scales, valid, early);
     return launch_pdl(quantize_rows_vec<TPR, false>, dim3(grid), dim3(kThreads), 0, stream,
-                      x, rows, k, q, ldq, row_scales, valid);
+                      x, rows, k, q, ldq, row_scales, valid, early);
 }
 
 template <int TPR, int PER>
 cudaError_t launch_any_per(const float* x, uint32_t rows, uint32_t k, int8_t* q, uint32_t ldq,
-                           float* row_scales, int32_t* valid, cudaStream_t stream) {
+                           float* row_scales, int32_t* valid, cudaStream_t stream, bool early) {
     constexpr uint32_t kRowsPerCta = kThreads / TPR;
     return launch_pdl(quantize_rows_any<TPR, PER>, dim3((rows + kRowsPerCta - 1) / kRowsPerCta), dim3(kThreads), 0, stream,
-                      x, rows, k, q, ldq, row_scales, valid);
+                      x, rows, k, q, ldq, row_scales, valid, early);
 }
 template <int TPR>
 cudaError_t launch_any(const float* x, uint32_t rows, uint32_t k, int8_t* q, uint32_t ldq,
-                       float* row_scales, int32_t* valid, cudaStream_t stream) {
-    if (k <= (uint32_t)TPR * 4) return launch_any_per<TPR, 4>(x, rows, k, q, ldq, row_scales, valid, stream);
-    if (k <= (uint32_t)TPR * 8) return launch_any_per<TPR, 8>(x, rows, k, q, ldq, row_scales, valid, stream);
-    if (k <= (uint32_t)TPR * 16) return launch_any_per<TPR, 16>(x, rows, k, q, ldq, row_scales, valid, stream);
-    if (k <= (uint32_t)TPR * kMaxPerThread) return launch_any_per<TPR, kMaxPerThread>(x, rows, k, q, ldq, row_scales, valid, stream);
-    return launch_any_per<kThreads, 0>(x, rows, k, q, ldq, row_scales, valid, stream);   // (TPR is kThreads then)
+                       float* row_scales, int32_t* valid, cudaStream_t stream, bool early) {
+    if (k <= (uint32_t)TPR * 4) return launch_any_per<TPR, 4>(x, rows, k, q, ldq, row_scales, valid, stream, early);
+    if (k <= (uint32_t)TPR * 8) return launch_any_per<TPR, 8>(x, rows, k, q, ldq, row_scales, valid, stream, early);
+    if (k <= (uint32_t)TPR * 16) return launch_any_per<TPR, 16>(x, rows, k, q, ldq, row_scales, valid, stream, early);
+    if (k <= (uint32_t)TPR * kMaxPerThread) return launch_any_per<TPR, kMaxPerThread>(x, rows, k, q, ldq, row_scales, valid, stream, early);
+    return launch_any_per<kThreads, 0>(x, rows, k, q, ldq, row_scales, valid, stream, early);   // (TPR is kThreads then)
 }
 
 
@@ -565,30 +570,30 @@ uint32_t quantize_vec_threads(uint32_t rows, uint32_t k, bool norm) {
 }
 
 cudaError_t launch_quantize_rows(const float* x, uint32_t rows, uint32_t k, int8_t* q, uint32_t ldq,
-                                 float* row_scales, int32_t* valid, cudaStream_t stream) {
+                                 float* row_scales, int32_t* valid, cudaStream_t stream, bool early) {
     if (rows == 0) return cudaSuccess;
     const bool vec = (k % 4 == 0) && (ldq % 4 == 0) && ((uintptr_t)x % 16 == 0) && ((uintptr_t)q % 4 == 0);
     if (!vec) {
         // one warp per row where that alone fills the chip, more threads per row (and loads in flight) otherwise
         const uint32_t tpr = quantize_any_threads(rows, k);
-        if (tpr == 32) return launch_any<32>(x, rows, k, q, ldq, row_scales, valid, stream);
-        if (tpr == 64) return launch_any<64>(x, rows, k, q, ldq, row_scales, valid, stream);
-        if (tpr == 128) return launch_any<128>(x, rows, k, q, ldq, row_scales, valid, stream);
-        return launch_any<256>(x, rows, k, q, ldq, row_scales, valid, stream);
+        if (tpr == 32) return launch_any<32>(x, rows, k, q, ldq, row_scales, valid, stream, early);
+        if (tpr == 64) return launch_any<64>(x, rows, k, q, ldq, row_scales, valid, stream, early);
+        if (tpr == 128) return launch_any<128>(x, rows, k, q, ldq, row_scales, valid, stream, early);
+        return launch_any<256>(x, rows, k, q, ldq, row_scales, valid, stream, early);
     }
     // Few long rows: a cluster of 2..8 CTAs per row (each thread then holds one or two float4)
     if (rows <= kClusterMaxRows && ldq / 4 >= 2u * kThreads && ldq / 4 <= 8u * kThreads * kMaxVecPerThread) {
         const uint32_t per = (ldq / 4 + kThreads - 1) / kThreads;   // float4 per thread with one CTA
-        if (per >= 8) return launch_cluster<8>(x, rows, k, q, ldq, row_scales, valid, stream);
-        if (per >= 4) return launch_cluster<4>(x, rows, k, q, ldq, row_scales, valid, stream);
-        return launch_cluster<2>(x, rows, k, q, ldq, row_scales, valid, stream);
+        if (per >= 8) return launch_cluster<8>(x, rows, k, q, ldq, row_scales, valid, stream, early);
+        if (per >= 4) return launch_cluster<4>(x, rows, k, q, ldq, row_scales, valid, stream, early);
+        return launch_cluster<2>(x, rows, k, q, ldq, row_scales, valid, stream, early);
     }
     switch (quantize_vec_threads(rows, k)) {
-        case 8: return launch_vec<8>(x, rows, k, q, ldq, row_scales, valid, stream);
-        case 32: return launch_vec<32>(x, rows, k, q, ldq, row_scales, valid, stream);
-        case 64: return launch_vec<64>(x, rows, k, q, ldq, row_scales, valid, stream);
-        case 128: return launch_vec<128>(x, rows, k, q, ldq, row_scales, valid, stream);
-        default: return launch_vec<256>(x, rows, k, q, ldq, row_scales, valid, stream);
+        case 8: return launch_vec<8>(x, rows, k, q, ldq, row_scales, valid, stream, early);
+        case 32: return launch_vec<32>(x, rows, k, q, ldq, row_scales, valid, stream, early);
+        case 64: return launch_vec<64>(x, rows, k, q, ldq, row_scales, valid, stream, early);
+        case 128: return launch_vec<128>(x, rows, k, q, ldq, row_scales, valid, stream, early);
+        default: return launch_vec<256>(x, rows, k, q, ldq, row_scales, valid, stream, early);
     }
 }
 
