@@ -106,7 +106,7 @@ typedef struct VxbPlanQuery {
     uint32_t sm_count;       /* SMs of the device (148 on a B200) */
     uint32_t pair_clusters;  /* co-resident clusters of two the device grants the pair kernel (0: none) */
     uint32_t out_store_aligned; /* the output's (and every peer buffer's) base, row pitch and width are multiples of 16 bytes \
-                                   (TMA tile stores possible) */
+                                   (TMA tile stores possible); for int8 without peers the base and the row pitch */
 } VxbPlanQuery;
 
 /* Per-row quantizer (K1) chosen for calls that start from fp32 activations. */

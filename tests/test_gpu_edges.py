@@ -297,6 +297,32 @@ def test_rows_past_64_in_tiles(torch, ctx, rows, k, n):
     weight.close()
 
 
+@pytest.mark.parametrize("rows,k,n", [(65, 1536, 2050), (97, 1100, 1022), (128, 100, 3090), (80, 1100, 66)])
+def test_rows_past_64_in_the_decode_kernel(torch, ctx, rows, k, n):
+    """65 to 128 rows where unaligned outputs and the SiLU * Mul tail keep the decode kernel: equal to the tile kernels'."""
+    from volvoxai_b200 import w8a8
+    c = wl.single_linear(rows=rows, k=k, n=n, seed=rows + k + n)
+    weight = w8a8.Weight.from_i8(ctx, c["w"], c["ws"], bias_f32=c["bias"], bias_i32=np.arange(n, dtype=np.int32) * 5 - 300)
+    x = dev(torch, c["x"])
+    res = torch.randn((rows, n), device="cuda")
+    tiles = ctx.linear_f32(weight, x, route=w8a8.ROUTE_TCGEN05)
+
+    def decoded(y):
+        assert "decode-rows" in w8a8.last_route()
+        return y
+
+    assert torch.equal(decoded(ctx.linear_f32(weight, x)), tiles)
+    assert torch.equal(decoded(ctx.linear_acc_i32(weight, x)), ctx.linear_acc_i32(weight, x, route=w8a8.ROUTE_TCGEN05))
+    assert torch.equal(decoded(ctx.linear_f32_fused(weight, x, residual=res)), tiles + res)
+    s = decoded(ctx.linear_f32_fused(weight, x, silu_mul=True)).double()
+    g, u = tiles[:, 0::2].double(), tiles[:, 1::2].double()
+    y = g / (1.0 + torch.exp(-g)) * u
+    assert (s - y).abs().le(1e-6 * y.abs() + 1e-30).all()      # four roundings and an expf of at most 2 ulp
+    y8 = ctx.linear_i8(weight, x, 0.1, -5)
+    assert torch.equal(y8, ctx.linear_i8(weight, x, 0.1, -5, route=w8a8.ROUTE_TCGEN05))
+    weight.close()
+
+
 @pytest.mark.parametrize("captured", [False, True])
 def test_small_calls_back_to_back(torch, ctx, captured):
     """Calls on both sides of the line up to which the quantizer lets its GEMM in before its own wait, and single-launch

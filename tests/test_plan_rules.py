@@ -17,6 +17,24 @@ def test_rows_past_64_keep_the_decode_kernel_for_small_weights_only(rows, k, n, 
         assert (pick(rows, k, n, epilogue=epilogue)["id"] == "DECODE_ROWS") == decode
 
 
+@pytest.mark.parametrize("kw,inside,outside", [
+    ({"out_store_aligned": False}, [(128, 1536, 4736), (80, 1536, 9472), (65, 100, 5000)], [(65, 1537, 1024), (81, 64, 4737), (80, 64, 9473)]),
+    ({"out_store_aligned": False, "epilogue": _lib.EPI_ACC}, [(124, 1152, 3224)], [(66, 1537, 64)]),
+    ({"out_store_aligned": False, "epilogue": _lib.EPI_I8}, [(80, 768, 4736), (128, 512, 4736)], [(128, 512, 4737), (65, 512, 4737), (80, 896, 3073), (65, 1025, 64)]),
+    ({"out_store_aligned": True, "epilogue": _lib.EPI_I8}, [(128, 1024, 3072)], [(65, 128, 3073)]),
+    ({"fused_tail": 2}, [(128, 1536, 4736), (96, 576, 9472)], [(97, 1536, 4738), (65, 1664, 1024), (65, 64, 9474)]),
+    ({"fused_tail": 2, "out_store_aligned": False}, [(96, 1024, 6000)], [(97, 1024, 6000)]),
+])
+def test_rows_past_64_by_what_the_output_costs_in_tiles(kw, inside, outside):
+    """Unaligned outputs and the SiLU * Mul tail keep the decode kernel further than the small weights above."""
+    for shape in inside:
+        assert pick(*shape, **kw)["id"] == "DECODE_ROWS", shape
+    for shape in outside:
+        assert pick(*shape, **kw)["id"] != "DECODE_ROWS", shape
+    for rows, k, n in inside + outside:
+        assert pick(64, k, n, **kw)["id"] == "DECODE_ROWS" and pick(129, k, n, **kw)["id"] != "DECODE_ROWS"
+
+
 @pytest.mark.parametrize("rows,k,n,want", [(512, 4096, 4096, "TCGEN05_PAIR_NARROW"), (1024, 4096, 4096, "TCGEN05"), (2048, 4096, 4096, "TCGEN05_PAIR"),
                                            (512, 1536, 4096, "TCGEN05"), (512, 1537, 4096, "TCGEN05_PAIR_NARROW")])
 def test_long_k_takes_the_cheapest_waves(rows, k, n, want):

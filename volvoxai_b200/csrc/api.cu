@@ -314,8 +314,9 @@ VxbPlanQuery plan_query(const VxbContext* ctx, const VxbWeight* w, uint32_t rows
     query.requested_route = requested; query.n_peers = epi.n_peers;
     query.fused_tail = (epi.residual ? 1u : 0u) | (epi.act ? 2u : 0u);
     // TMA tile stores clip at the matrix edge in units of 16 bytes: the width must be a multiple of four 32-bit columns too
-    query.out_store_aligned = (epi.mode != kEpiI8 && !((uintptr_t)epi.out & 15u) && !(epi.ld & 3u) &&
-                               !((epi.act ? w->d_out >> 1 : w->d_out) & 3u)) ? 1u : 0u;
+    const bool base_aligned = !((uintptr_t)epi.out & 15u);
+    query.out_store_aligned = (epi.mode == kEpiI8 ? base_aligned && !(epi.ld & 15u)
+                                                  : base_aligned && !(epi.ld & 3u) && !((epi.act ? w->d_out >> 1 : w->d_out) & 3u)) ? 1u : 0u;
     if (epi.mode == kEpiI8 && epi.n_peers) {
         bool aligned = !((uintptr_t)epi.out & 15u) && !(epi.ld & 15u) && !(w->d_out & 15u) && tunables().gather_tma;
         for (uint32_t p = 0; p < epi.n_peers; p++) aligned = aligned && !((uintptr_t)epi.peer_out[p] & 15u);

@@ -151,6 +151,27 @@ void plan_quantizer(const VxbPlanQuery& q, VxbLaunchPlan* p) {
     p->quantizer_grid = ceil_div(q.rows, 256 / tpr);
 }
 
+// 65 to 128 rows in the decode kernel (128 token slots, 128 clocks an MMA: its time grows with the rows, the 32-channel
+// pieces of a CTA's share and K) instead of tiles, whose time is one wave and how the output leaves them: TMA stores for
+// aligned 32-bit words, 16 bytes a lane for aligned int8, the warps' store tiles for unaligned rows, eight warps for the
+// SiLU * Mul tail.  us replayed from a graph, decode / tiles, at K -> N and 65, 96 and 128 rows (N 3072, 6144 and 11008:
+// one, two and three pieces):
+//   unaligned fp32 512 -> 3072 8.2/11.3 8.9/11.4 9.8/11.7;  1024 -> 6144 11.8/12.5 13.5/12.6 15.6/13.0;  2048 -> 1024 13.9/11.0 14.7/11.1 15.6/11.2
+//   SiLU * Mul     512 -> 3072 9.2/14.6 10.3/14.9 11.8/15.3;  1024 -> 6144 14.0/15.9 16.1/16.2 19.4/16.4;  1536 -> 11008 19.9/17.5 23.4/17.7 27.4/18.0
+//   unaligned int8 256 -> 3072 7.8/10.0 8.7/10.1 10.2/10.2;  512 -> 3072 9.1/10.8 10.1/10.7 11.5/10.9;  512 -> 6144 12.2/10.7 14.4/10.8 17.1/10.9
+//   aligned fp32   256 -> 1024 6.7/6.9 7.4/7.0 8.0/7.5;  512 -> 3072 8.1/7.7 8.9/7.8 9.8/8.2;  1024 -> 3072 9.8/8.9 10.7/9.3 11.5/9.4;
+//                  1024 -> 6144 12.1/9.0 13.3/9.2 15.5/9.5
+// (K above 1536 goes to the paired tiles, in half of the decode kernel's time.)  The last line of the rule, all outputs up
+// to K 1024 and N 3072, is older than the fast stores of the aligned ones, which are past their crossing there.
+bool decode_past_64_rows(const VxbPlanQuery& q) {
+    const uint32_t kpad = round_up(q.k, kKAlign);
+    const uint64_t work = (uint64_t)q.rows * ceil_div(ceil_div(q.n, q.sm_count ? q.sm_count : 148u), 32u);
+    if (q.rows > 128 || kpad > VXB_WIDE_MAX_KPAD) return false;
+    if ((q.fused_tail & 2u) && work <= 192) return true;
+    if (!q.out_store_aligned && (q.epilogue == VXB_EPI_I8 ? work <= 128 && q.rows * kpad <= 65536u : work <= 160)) return true;
+    return kpad <= 1024 && q.n <= 3072;
+}
+
 }  // namespace
 
 extern "C" {
@@ -209,10 +230,7 @@ int vxb_plan(const VxbPlanQuery* query, VxbLaunchPlan* out, char* why, uint32_t 
             if (q.rows > 128 && tiles >= 2u * sms && (uint64_t)q.n_peers * 3424u <= round_up(q.k, kKAlign) &&
                 admitted(kVariants[VXB_VARIANT_TCGEN05_PAIR], q, unused, sizeof unused)) chosen = VXB_VARIANT_TCGEN05_PAIR;
         }
-        else if (q.rows <= 64 || (q.rows <= 128 && round_up(q.k, kKAlign) <= 1024u && q.n <= 3072u)) {
-            // (65 to 128 rows are 128 token slots, and an MMA of the decode kernel takes its 128 clocks whatever its
-            // channels: 128 x 4096 -> 4096 20.9 us against 16.2 in tiles of 128 x 256, 128 x 1024 -> 6144 13.3 against
-            // 9.1, 128 x 1024 -> 3072 9.5 against 9.0)
+        else if (q.rows <= 64 || decode_past_64_rows(q)) {
             chosen = VXB_VARIANT_DECODE_ROWS;
             char unused[8];
             // one or two fp32 rows: the single-launch form.  From three rows on every CTA repeating the
