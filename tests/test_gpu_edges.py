@@ -185,6 +185,24 @@ def test_quantize_linear_scales_and_extremes(torch, ctx, oracle, scale, unsigned
     assert np.array_equal(got, oracle.quantize_linear(x, float(s), zero, unsigned))
 
 
+@pytest.mark.parametrize("count", [1, 15, 16, 17, 255, 257, 4095, 4096, 4097, 8191, 12289])
+@pytest.mark.parametrize("lead", [0, 1, 3])
+def test_boundary_ops_last_blocks_and_unaligned_inputs(torch, ctx, oracle, count, lead):
+    """Counts around a thread's 16 elements and a block's 4096, inputs `lead` elements off."""
+    rng = np.random.default_rng(count + lead)
+    x = (rng.standard_normal(count + lead) * 3).astype(np.float32)
+    xd, x = dev(torch, x)[lead:], x[lead:]
+    for scale, zero, unsigned in ((0.05, -3, False), (1e-12, 3, True)):
+        assert np.array_equal(ctx.quantize_linear(xd, scale, zero, unsigned).cpu().numpy(), oracle.quantize_linear(x, scale, zero, unsigned))
+    for dtype, lo, hi, zero in ((np.int8, -128, 128, -7), (np.uint8, 0, 256, 130)):
+        c = rng.integers(lo, hi, size=count + lead).astype(dtype)
+        cd, c = dev(torch, c)[lead:], c[lead:]
+        assert np.array_equal(bits(ctx.dequantize_linear(cd, 0.031, zero).cpu().numpy()), bits(oracle.dequantize_linear(c, 0.031, zero)))
+        for unsigned in (False, True):
+            assert np.array_equal(ctx.requantize_linear(cd, 0.031, zero, 0.05, 4, unsigned).cpu().numpy(),
+                                  oracle.requantize_linear(c, 0.031, zero, 0.05, 4, unsigned))
+
+
 @pytest.mark.parametrize("group", [32, 64, 128, 256])
 @pytest.mark.parametrize("rows,k,n", [(5, 300, 1), (8, 640, 129), (9, 4096, 100), (17, 1283, 300), (33, 896, 64), (64, 2176, 257),
                                       (7, 272, 10000), (40, 384, 19200), (12, 4224, 70), (5, 2048, 4200)])
