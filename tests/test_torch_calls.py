@@ -1,12 +1,17 @@
 """The native form of the device calls (csrc/torch_calls.cpp) without a GPU: whatever torch refuses comes back as a Python
 exception, whatever the library declines as W8A8Error, and what is not a torch tensor goes through ctypes."""
+import os
+import subprocess
+
 import numpy as np
 import pytest
 import torch
 
-from volvoxai_b200 import w8a8
+from volvoxai_b200 import build, w8a8
 
-calls = pytest.importorskip("volvoxai_b200._torch_calls")
+if not build.torch_calls_built():
+    pytest.skip("_torch_calls.so is not built for this Python and torch", allow_module_level=True)
+from volvoxai_b200 import _torch_calls as calls  # noqa: E402  (a module that does not load fails here)
 
 
 class Closed:
@@ -55,3 +60,41 @@ def test_only_torch_tensors_take_the_native_form():
     assert w8a8._calls(torch.zeros(1)) is calls
     assert w8a8._calls(torch.nn.Parameter(torch.zeros(1))) is calls
     assert w8a8._calls(np.zeros(1)) is None and w8a8._calls(None) is None
+
+
+@pytest.fixture
+def scratch(tmp_path, monkeypatch):
+    """build.py with the module elsewhere, and w8a8.py as before its first call."""
+    monkeypatch.setattr(build, "TORCH_CALLS", str(tmp_path / "_torch_calls.so"))
+    monkeypatch.setattr(w8a8, "_torch_calls", False)
+    return tmp_path
+
+
+def put(scratch, key):
+    (scratch / "_torch_calls.so").write_bytes(b"...built for " + key.encode() + b"\0...")
+
+
+def test_the_library_builds_where_the_module_cannot(scratch, monkeypatch, capsys):
+    put(scratch, "another")
+    monkeypatch.setattr(subprocess, "run", lambda *a, **k: subprocess.CompletedProcess(a, 1, "", "no Python.h"))
+    assert build.build_torch_calls() is None and "no Python.h" in capsys.readouterr().err
+    assert os.listdir(scratch) == []
+    def missing(*a, **k):
+        raise FileNotFoundError("g++")
+    monkeypatch.setattr(subprocess, "run", missing)
+    assert build.build_torch_calls(force=True) is None
+    assert w8a8._calls(torch.zeros(1)) is None
+
+
+@pytest.mark.parametrize("same", [True, False])
+def test_a_module_for_another_torch_is_not_used(scratch, monkeypatch, same):
+    put(scratch, build.torch_calls_key())
+    if not same:
+        monkeypatch.setattr(torch, "__version__", "0.1")
+    assert build.torch_calls_built() == same
+    assert (w8a8._calls(torch.zeros(1)) is calls) == same
+    built = []
+    os.utime(build.TORCH_CALLS)
+    monkeypatch.setattr(subprocess, "run", lambda *a, **k: built.append(a) or subprocess.CompletedProcess(a, 0, "", ""))
+    build.build_torch_calls()
+    assert bool(built) != same and build.torch_calls_built() == same      # (the stand-in compiler leaves no module)

@@ -60,25 +60,49 @@ TORCH_CALLS = os.path.join(PKG, "_torch_calls.so")
 TORCH_CALLS_SRC = os.path.join(CSRC, "torch_calls.cpp")
 
 
-def build_torch_calls(force: bool = False) -> str:
-    """Builds _torch_calls.so (w8a8.py's device calls in native code) against the running Python's torch."""
-    deps = [TORCH_CALLS_SRC, os.path.join(ROOT, "include", "vxb200_w8a8.h")]
-    if not force and os.path.exists(TORCH_CALLS) and all(os.path.getmtime(d) <= os.path.getmtime(TORCH_CALLS) for d in deps):
-        return TORCH_CALLS
-    import sysconfig
-
+def torch_calls_key() -> str:
+    """The running Python and torch, whose binary interfaces _torch_calls.so is built against."""
     import torch
-    from torch.utils import cpp_extension
-    includes = [f"-isystem{p}" for p in cpp_extension.include_paths() + [sysconfig.get_paths()["include"]]]
-    torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
-    cmd = ["g++", "-std=c++20", "-O2", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
-           *includes, "-o", TORCH_CALLS, TORCH_CALLS_SRC, "-L", PKG, "-l:libvxb200.so", "-Wl,-rpath,$ORIGIN",
-           "-L", torch_lib, "-lc10", "-ltorch_cpu", "-ltorch_python"]
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if res.returncode != 0:
-        sys.stderr.write(res.stdout + res.stderr)
-        raise RuntimeError("g++ failed building _torch_calls.so")
-    return TORCH_CALLS
+    return f"{sys.implementation.cache_tag} torch {torch.__version__}"
+
+
+def torch_calls_built() -> bool:
+    """Whether _torch_calls.so is there and is for the running Python and torch: the module carries the key it was built
+    with (kBuiltFor in torch_calls.cpp), which is looked for in the file so that a module for another torch is never loaded."""
+    try:
+        with open(TORCH_CALLS, "rb") as f:
+            return f"built for {torch_calls_key()}\0".encode() in f.read()
+    except OSError:
+        return False
+
+
+def build_torch_calls(force: bool = False) -> str | None:
+    """Builds _torch_calls.so (w8a8.py's device calls in native code) against the running Python's torch.  The library needs
+    none of what this needs - torch and its headers, Python's headers, a C++20 compiler - and w8a8.py has a ctypes form of
+    the same calls, so a failure is reported and is not an error: returns None then, and leaves no module behind."""
+    deps = [TORCH_CALLS_SRC, os.path.join(ROOT, "include", "vxb200_w8a8.h")]
+    try:
+        if not force and torch_calls_built() and all(os.path.getmtime(d) <= os.path.getmtime(TORCH_CALLS) for d in deps):
+            return TORCH_CALLS
+        if os.path.exists(TORCH_CALLS):
+            os.remove(TORCH_CALLS)
+        import sysconfig
+
+        import torch
+        from torch.utils import cpp_extension
+        includes = [f"-isystem{p}" for p in cpp_extension.include_paths() + [sysconfig.get_paths()["include"]]]
+        torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+        cmd = ["g++", "-std=c++20", "-O2", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+               f'-DVXB_BUILT_FOR="{torch_calls_key()}"',
+               *includes, "-o", TORCH_CALLS, TORCH_CALLS_SRC, "-L", PKG, "-l:libvxb200.so", "-Wl,-rpath,$ORIGIN",
+               "-L", torch_lib, "-lc10", "-ltorch_cpu", "-ltorch_python"]
+        res = subprocess.run(cmd, capture_output=True, text=True)
+        if res.returncode != 0:
+            raise RuntimeError(res.stdout + res.stderr)
+        return TORCH_CALLS
+    except (ImportError, OSError, RuntimeError) as e:
+        sys.stderr.write(f"_torch_calls.so was not built (the ctypes calls serve): {e}\n")
+        return None
 
 
 PROVIDER_LIB = os.path.join(PKG, "libvxb200_provider.so")

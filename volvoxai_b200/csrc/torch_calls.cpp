@@ -19,6 +19,9 @@
 
 namespace {
 
+// The Python and torch of the build, which build.py looks for in the file before the module is loaded.
+__attribute__((used)) const char kBuiltFor[] = "built for " VXB_BUILT_FOR;
+
 using at::Tensor;
 
 // Arguments of one call, read left to right; `bad` is set (with a Python error) by the first that does not fit.

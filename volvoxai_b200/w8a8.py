@@ -53,17 +53,26 @@ def _ptr(a) -> C.c_void_p:
 _torch_calls = False   # not looked for yet
 
 
+def _load_calls():
+    """(the native form of the device calls, csrc/torch_calls.cpp; torch's tensor type), or None where there is no torch or
+    no module for this Python and torch.  A module that is for them and does not load is an error."""
+    try:
+        import torch
+    except ImportError:
+        return None
+    from . import build
+    if not build.torch_calls_built():
+        return None
+    from . import _torch_calls as module
+    return module, torch.Tensor
+
+
 def _calls(x):
-    """The native form of the device calls (csrc/torch_calls.cpp) for a torch tensor; None for anything else, or where
-    the module was not built: the ctypes form below serves then, with the same results."""
+    """The native form of the device calls for a torch tensor; None for anything else, or without the module: the ctypes
+    form below serves then, with the same results."""
     global _torch_calls
     if _torch_calls is False:
-        try:
-            import torch
-            from . import _torch_calls as module
-            _torch_calls = (module, torch.Tensor)
-        except ImportError:
-            _torch_calls = None
+        _torch_calls = _load_calls()
     return _torch_calls[0] if _torch_calls is not None and isinstance(x, _torch_calls[1]) else None
 
 
