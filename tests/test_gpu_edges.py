@@ -341,6 +341,43 @@ def test_rows_past_64_in_the_decode_kernel(torch, ctx, rows, k, n):
     weight.close()
 
 
+def test_native_and_ctypes_calls_agree(torch, ctx, monkeypatch):
+    """The eight device calls in both forms, and with outputs, residuals and norm weights that are not torch's."""
+    from tests.test_torch_calls import Memory
+    from volvoxai_b200 import w8a8
+    rows, k, n = 9, 300, 66
+    c = wl.single_linear(rows=rows, k=k, n=n, seed=1)
+    weight = w8a8.Weight.from_i8(ctx, c["w"], c["ws"], bias_f32=c["bias"], bias_i32=np.arange(n, dtype=np.int32))
+    x, res = dev(torch, c["x"]), torch.randn((rows, n), device="cuda")
+    gamma = torch.rand(k, device="cuda") + 0.5
+    q = torch.randint(-128, 128, (rows, k), dtype=torch.int8, device="cuda")
+    outs = {"y": torch.empty((rows, n), device="cuda"), "norm": torch.empty((rows, k), device="cuda")}
+
+    def memory(t):
+        return Memory(t.data_ptr(), t.stride(0))
+
+    def into(call):
+        for t in outs.values():
+            t.zero_()
+        call()
+        return torch.cat([t.flatten() for t in outs.values()])
+
+    calls = [lambda: ctx.linear_f32(weight, x), lambda: ctx.linear_f32_fused(weight, x, residual=res), lambda: ctx.linear_f32_fused(weight, x, silu_mul=True),
+             lambda: ctx.rmsnorm_linear_f32_fused(weight, x, gamma, 1e-6), lambda: ctx.linear_i8(weight, x, 0.1, 3),
+             lambda: ctx.qlinear_device(weight, q, 0.05, -3, 0.5, 4, out_unsigned=True), lambda: ctx.quantize_linear(x, 0.1, 5),
+             lambda: ctx.dequantize_linear(q, 0.1, 5), lambda: ctx.requantize_linear(q, 0.1, 5, 0.2, 7, unsigned=True)]
+    native = [call() for call in calls]
+    native.append(into(lambda: ctx.rmsnorm_linear_f32_fused(weight, x, gamma, 1e-6, norm_out=outs["norm"], out=outs["y"])))
+    assert torch.equal(native[-1], into(lambda: ctx.rmsnorm_linear_f32_fused(weight, x, memory(gamma), 1e-6, norm_out=memory(outs["norm"]), out=memory(outs["y"]))))
+    assert torch.equal(into(lambda: ctx.linear_f32_fused(weight, x, residual=memory(res), out=outs["y"]))[:rows * n], native[1].flatten())
+    assert torch.equal(into(lambda: ctx.linear_f32(weight, x, out=memory(outs["y"])))[:rows * n], native[0].flatten())
+    monkeypatch.setattr(w8a8, "_torch_calls", None)
+    for call, want in zip(calls, native):
+        got = call()
+        assert got.dtype == want.dtype and torch.equal(got, want)
+    weight.close()
+
+
 @pytest.mark.parametrize("captured", [False, True])
 def test_small_calls_back_to_back(torch, ctx, captured):
     """Calls on both sides of the line up to which the quantizer lets its GEMM in before its own wait, and single-launch

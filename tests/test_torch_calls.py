@@ -62,6 +62,35 @@ def test_only_torch_tensors_take_the_native_form():
     assert w8a8._calls(np.zeros(1)) is None and w8a8._calls(None) is None
 
 
+class Memory:
+    """Not a torch tensor, but with a device pointer and a row pitch."""
+    def __init__(self, at=0, pitch=8):
+        self.at, self.pitch = at, pitch
+
+    def data_ptr(self):
+        return self.at
+
+    def stride(self, dim):
+        return self.pitch
+
+
+def test_calls_with_other_memory_go_through_ctypes():
+    """An output, residual, norm weight or norm output that is not torch's: declined by the library here (null handles),
+    where the native form would refuse the argument."""
+    x, other = torch.zeros(2, 8), Memory()
+    context, weight = Closed(), Closed()
+    weight.d_out, context._L, context.handle, weight.handle = 8, w8a8._lib.load(), None, None
+    f = w8a8.Context
+    for call in (lambda: f.linear_f32(context, weight, x, out=other), lambda: f.linear_i8(context, weight, x, 0.1, out=other),
+                 lambda: f.linear_f32_fused(context, weight, x, residual=other), lambda: f.linear_f32_fused(context, weight, x, out=other),
+                 lambda: f.rmsnorm_linear_f32_fused(context, weight, x, other, 1e-6),
+                 lambda: f.rmsnorm_linear_f32_fused(context, weight, x, x[0], 1e-6, norm_out=other),
+                 lambda: f.rmsnorm_linear_f32_fused(context, weight, x, None, 1e-6)):
+        with pytest.raises(w8a8.W8A8Error):
+            call()
+    assert w8a8._calls(x, None, x) is calls and w8a8._calls(x, None, other) is None
+
+
 @pytest.fixture
 def scratch(tmp_path, monkeypatch):
     """build.py with the module elsewhere, and w8a8.py as before its first call."""

@@ -114,7 +114,7 @@ PyObject* rmsnorm_linear_f32_fused(PyObject*, PyObject* const* args, Py_ssize_t 
     Args a{args, n};
     auto* ctx = a.handle<VxbContext>(); auto* w = a.handle<VxbWeight>();
     const Tensor* x = a.tensor(); const long long width = a.integer(); const Tensor* out = a.tensor(true);
-    const Tensor* g = a.tensor(); const double eps = a.number(); const Tensor* norm_out = a.tensor(true); const int silu = (int)a.integer();
+    const Tensor* g = a.tensor(true); const double eps = a.number(); const Tensor* norm_out = a.tensor(true); const int silu = (int)a.integer();
     if (a.bad) return nullptr;
     const int64_t rows = x->size(0);
     return result(out, [&] { return matrix(*x, rows, width, at::kFloat); }, [&, in = at_of(x), gp = at_of(g), no = at_of(norm_out)](void* y, uint32_t ld) {

@@ -67,13 +67,18 @@ def _load_calls():
     return module, torch.Tensor
 
 
-def _calls(x):
-    """The native form of the device calls for a torch tensor; None for anything else, or without the module: the ctypes
-    form below serves then, with the same results."""
+def _calls(x, *others):
+    """The native form of the device calls where every tensor of the call (None: not given) is torch's; None for anything
+    else with a device pointer, or without the module: the ctypes form below serves then, with the same results."""
     global _torch_calls
     if _torch_calls is False:
         _torch_calls = _load_calls()
-    return _torch_calls[0] if _torch_calls is not None and isinstance(x, _torch_calls[1]) else None
+    if _torch_calls is None or not isinstance(x, _torch_calls[1]):
+        return None
+    for t in others:
+        if t is not None and not isinstance(t, _torch_calls[1]):
+            return None
+    return _torch_calls[0]
 
 
 def _done(result):
@@ -246,7 +251,7 @@ class Context:
                                  norm_out=None, out=None):
         """RMSNorm -> quantize -> linear (+ silu(gate) * up over interleaved channel pairs)."""
         width = w.d_out // 2 if silu_mul else w.d_out
-        native = _calls(x)
+        native = _calls(x, norm_weight, norm_out, out)
         if native is not None:
             return _done(native.rmsnorm_linear_f32_fused(self._h, w._h, x, width, out, norm_weight, epsilon, norm_out, 1 if silu_mul else 0))
         import torch
@@ -259,7 +264,7 @@ class Context:
         return out
 
     def linear_f32(self, w: "Weight", x, out=None, route: int = ROUTE_AUTO):
-        native = _calls(x)
+        native = _calls(x, out)
         if native is not None:
             return _done(native.linear_f32(self._h, w._h, x, w.d_out, out, route))
         import torch
@@ -274,7 +279,7 @@ class Context:
         """fp32 linear with a fused tail: + residual, or silu(gate) * up over interleaved channel
         pairs (output d_out / 2 wide)."""
         width = w.d_out // 2 if silu_mul else w.d_out
-        native = _calls(x)
+        native = _calls(x, residual, out)
         if native is not None:
             return _done(native.linear_f32_fused(self._h, w._h, x, width, out, residual, 1 if silu_mul else 0))
         import torch
@@ -289,7 +294,7 @@ class Context:
 
     def linear_i8(self, w: "Weight", x, out_scale: float, out_zero: int = 0, out=None,
                   route: int = ROUTE_AUTO):
-        native = _calls(x)
+        native = _calls(x, out)
         if native is not None:
             return _done(native.linear_i8(self._h, w._h, x, w.d_out, out, out_scale, int(out_zero), route))
         import torch
