@@ -205,7 +205,7 @@ def test_boundary_ops_last_blocks_and_unaligned_inputs(torch, ctx, oracle, count
 
 @pytest.mark.parametrize("group", [32, 64, 128, 256])
 @pytest.mark.parametrize("rows,k,n", [(5, 300, 1), (8, 640, 129), (9, 4096, 100), (17, 1283, 300), (33, 896, 64), (64, 2176, 257),
-                                      (7, 272, 10000), (40, 384, 19200), (12, 4224, 70), (5, 2048, 4200)])
+                                      (7, 272, 10000), (40, 384, 19200), (12, 4224, 70), (5, 2048, 4200), (3, 8200, 1540)])
 def test_grouped_few_rows(torch, ctx, oracle, group, rows, k, n):
     """Every token-slot count and both tile heights of the few-row kernel: ragged channels, a last stage half empty, a
     last group cut short, more tiles than SMs; rows one past a slot count take the next one."""

@@ -64,3 +64,9 @@ def test_quantizer_threads_per_row(rows, k, per_row):
     """Doubled while the launch stays within 256 threads per SM and a thread keeps a float4."""
     plan = pick(rows, k, 4096, fp32_input=True)
     assert plan["quantizer"] == 2 and plan["quantizer_grid"] == -(-rows // (256 // per_row))
+
+
+@pytest.mark.parametrize("rows,k,n,want", [(4, 8192, 1536, "GEMV_GROUPED"), (3, 8192, 1537, "GROUPED_TCGEN05"), (4, 8191, 4000, "GEMV_GROUPED"), (4, 14336, 2048, "GROUPED_TCGEN05"),
+                                           (2, 14336, 4096, "GEMV_GROUPED"), (4, 8191, 4097, "GROUPED_TCGEN05")])
+def test_three_and_four_grouped_rows(rows, k, n, want):
+    assert pick(rows, k, n, weight_kind=_lib.WEIGHT_GROUPED, group_size=128)["id"] == want

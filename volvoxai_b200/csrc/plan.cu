@@ -210,11 +210,14 @@ int vxb_plan(const VxbPlanQuery* query, VxbLaunchPlan* out, char* why, uint32_t 
     } else if (grouped) {
         if (q.epilogue != VXB_EPI_F32) return refuse(why, why_bytes, "weights with grouped scales produce fp32 output only");
         if (q.fused_tail) return refuse(why, why_bytes, "weights with grouped scales have no fused epilogue");
-        // decode: a warp per channel streams the weights once (over the 4-bit words when they were kept);
-        // from three rows on the tensor-core kernel is faster at large weights
+        // decode: a warp per channel streams the weights once (over the 4-bit words when they were kept); from three rows on
+        // the tensor-core kernel is faster at large weights, and at fewer bytes where K is long and the GEMV's blocks are more
+        // than half of the SMs (four rows, G = 128, from a graph / in a stream, us, GEMV and tiles: 8192 -> 1024 12.8/13.6 and
+        // 14.7/15.4, 8192 -> 2000 18.0/18.6 and 14.8/15.5, 8192 -> 4000 24.0/19.1 and 15.0/15.8, 11008 -> 2048 23.5/17.7 and
+        // 18.6/19.3)
         const uint64_t weight_bytes = (uint64_t)round_up(q.k, kKAlign) * q.n;
         if (q.rows <= 2 && q.weight_kind == VXB_WEIGHT_W4_WORDS) chosen = VXB_VARIANT_GEMV_W4_GROUPED;
-        else if (q.rows <= 2 || (q.rows <= 4 && weight_bytes <= (32ull << 20))) chosen = VXB_VARIANT_GEMV_GROUPED;
+        else if (q.rows <= 2 || (q.rows <= 4 && weight_bytes <= (32ull << 20) && !(q.k >= 8192 && q.n > 1536))) chosen = VXB_VARIANT_GEMV_GROUPED;
         else chosen = VXB_VARIANT_GROUPED_TCGEN05;
         if (!admitted(kVariants[chosen], q, why, why_bytes)) return 0;
     } else {
