@@ -58,8 +58,8 @@ def test_quantizer_elements_per_thread(torch, ctx, oracle, rows, k):
 @pytest.mark.parametrize("n", [1, 3, 31, 33, 62, 64, 66, 97, 129, 250, 257, 514])
 @pytest.mark.parametrize("rows,lead,extra", [(129, 0, 0), (161, 1, 2), (300, 2, 5), (140, 16, 32), (131, 4, 8)])
 def test_byte_outputs_on_any_boundary(torch, ctx, n, rows, lead, extra):
-    """int8 tiles whose rows start `lead` bytes into a row pitch of n + lead + extra: both tile kernels (and the
-    narrow tiles of the second), with bias and zero point, nothing written beside the window."""
+    """int8 tiles whose rows start `lead` bytes into a row pitch of n + lead + extra: both tile kernels, with bias and zero
+    point, nothing written beside the window."""
     from volvoxai_b200 import w8a8
     c = wl.single_linear(rows=rows, k=100, n=n, seed=n + rows)
     bias = np.arange(n, dtype=np.int32) * 37 - 900
@@ -136,6 +136,45 @@ def test_narrow_pair_tiles(torch, ctx, rows, k, n):
         y = call(w8a8.ROUTE_AUTO)
         assert "pair-narrow" in w8a8.last_route()
         assert torch.equal(y, call(w8a8.ROUTE_TCGEN05))
+    weight.close()
+
+
+@pytest.mark.parametrize("n", [1, 33, 64, 66, 129, 250])
+@pytest.mark.parametrize("rows,lead,extra", [(129, 0, 0), (161, 1, 2), (300, 2, 5), (140, 16, 32), (131, 4, 8)])
+def test_byte_outputs_of_the_narrow_tiles(torch, ctx, n, rows, lead, extra):
+    """The same windows from the 256 x 128 tiles, which the automatic route takes from padded K 1664 on."""
+    from volvoxai_b200 import w8a8
+    c = wl.single_linear(rows=rows, k=1600, n=n, seed=n + rows)
+    weight = w8a8.Weight.from_i8(ctx, c["w"], c["ws"], bias_i32=np.arange(n, dtype=np.int32) * 37 - 900)
+    x = dev(torch, c["x"])
+    wide = torch.full((rows, lead + n + extra), 99, dtype=torch.int8, device="cuda")
+    ctx.linear_i8(weight, x, 0.05, 3, out=wide[:, lead:lead + n])
+    assert "pair-narrow" in w8a8.last_route()
+    assert torch.equal(wide[:, lead:lead + n], ctx.linear_i8(weight, x, 0.05, 3, route=w8a8.ROUTE_SIMT))
+    assert (wide[:, :lead] == 99).all() and (wide[:, lead + n:] == 99).all()
+    weight.close()
+
+
+@pytest.mark.parametrize("rows,k,n,lead,want", [(512, 1664, 2050, 0, "pair-narrow"), (300, 2048, 388, 0, "pair-narrow"), (300, 2048, 386, 1, "pair-narrow"),
+                                                (512, 1700, 2048, 2, "pair-narrow"), (2048, 2048, 8192, 0, "tcgen05-pair-i8"),
+                                                (2048, 2048, 8192, 3, "tcgen05-pair-i8"), (4096, 256, 2560, 1, "tcgen05-pair-i8"),
+                                                (4090, 256, 2564, 2, "tcgen05-pair-i8")])
+def test_silu_tail_of_the_paired_tiles(torch, ctx, rows, k, n, lead, want):
+    """The SiLU * Mul tail of both paired tile widths, rows on 16 bytes, on 8 and on 4: bit-equal to the decode kernel's tail
+    (rows are independent of each other, 64 at a time take that kernel), nothing written beside the window."""
+    from volvoxai_b200 import w8a8
+    c = wl.single_linear(rows=rows, k=k, n=n, seed=rows + n)
+    weight = w8a8.Weight.from_i8(ctx, c["w"], c["ws"], bias_f32=c["bias"])
+    x = dev(torch, c["x"])
+    half = n // 2
+    wide = torch.full((rows, lead + half + (lead and 5)), 99.0, device="cuda")
+    ctx.linear_f32_fused(weight, x, silu_mul=True, out=wide[:, lead:lead + half])
+    assert want in w8a8.last_route(), w8a8.last_route()
+    assert (wide[:, :lead] == 99).all() and (wide[:, lead + half:] == 99).all()
+    for r in (0, 64, 128, 224, rows // 128 * 64, rows - 64):
+        part = ctx.linear_f32_fused(weight, x[r:r + 64], silu_mul=True)
+        assert "decode-rows" in w8a8.last_route()
+        assert torch.equal(wide[r:r + 64, lead:lead + half], part)
     weight.close()
 
 

@@ -676,7 +676,8 @@ def test_decoder_configuration_linear_shapes(torch, ctx, oracle, rows, k, n):
 def test_fused_residual_and_silu_mul(torch, ctx, oracle, rows, k, n):
     """linear + residual equals the oracle's fp32 output plus the residual, bit for bit; silu(gate) *
     up over interleaved channel pairs within the fp32 tolerance (the exponential is not part of the
-    bit-exact contract). Decode kernel (both epilogue forms), single-CTA and paired GEMM."""
+    bit-exact contract). Decode kernel (both epilogue forms) and single-CTA GEMMs, the last size with the
+    sixteen-warp tail (the paired GEMM's: test_silu_tail_of_the_paired_tiles)."""
     from volvoxai_b200 import w8a8
     c = wl.single_linear(rows=rows, k=k, n=n, seed=rows + n)
     ref = oracle.w8a8_linear(c["x"], c["w"], c["ws"], bias=c["bias"])["out"]
