@@ -110,11 +110,11 @@ __device__ __forceinline__ int32_t epi_i8(int32_t acc, float as, float ws, float
     return __float2int_rn(moved);
 }
 
-// Correctly rounded a / d for a constant divisor whose reciprocal rcp = RN(1/d) was
-// computed once: two Newton corrections with exact FMA residuals (the tail of the
-// IEEE division sequence, without the per-element reciprocal approximation and range
-// check). Valid - bit-identical to __fdiv_rn - when d's significand is not all ones and
-// a, d and a/d stay far from the fp32 exponent limits; the caller guards both.
+// Correctly rounded a / d for a constant divisor whose correctly rounded reciprocal rcp = RN(1/d) was computed once: the
+// quotient a * rcp corrected twice by exact fused residuals (P. Markstein, "Computation of elementary functions on the
+// IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990: with rcp correctly rounded such a correction gives the IEEE
+// quotient).  Valid - bit-identical to __fdiv_rn, checked over all divisors by vxb_selftest_div_const - when d's
+// significand is not all ones and a, d and a/d stay far from the fp32 exponent limits; the caller guards both.
 __device__ __forceinline__ float div_const(float a, float d, float rcp) {
     const float q0 = __fmul_rn(a, rcp);
     const float r0 = __fmaf_rn(-d, q0, a);

@@ -43,12 +43,17 @@ constexpr uint32_t kMaxTile = 256;         // channels per tile (UMMA N limit)
 // Two CTAs fit an SM (shared memory, registers and TMEM columns are all held to half of it), so
 // that the CTAs of the NEXT launch in the stream become resident while this launch still runs:
 // their prologue and the first ring-full of their weights overlap this launch's tail, and the
-// weight stream from HBM does not stop between back-to-back decode kernels.
+// weight stream from HBM does not stop between back-to-back decode kernels (prepared activations, the
+// single-launch form, and a quantizer that releases early).  Behind any other quantizer the launch before
+// has ended when this one starts.
 //
 // That only pays while a CTA's whole weight share is not much larger than the ring it can hold
 // in half an SM: then most of it is already in shared memory when the preceding kernel ends.
 // CTAs with more to stream run alone on their SM (kPair = false) with a ring twice as deep -
-// the stream rate follows the bytes in flight - and with up to eight MMA issuers.
+// the stream rate follows the bytes in flight - and with up to eight MMA issuers.  Behind a quantizer (us from a graph /
+// in a stream, in pairs and alone): 64 x 1024 -> 3072 6.8/7.2 and 7.5/8.2, 8 x 4096 -> 4096 10.1/9.8 and 10.0/10.5, 16 x
+// 2048 -> 4096 8.5/8.2 and 8.1/8.7, 32 x 2048 -> 5632 9.1/8.8 and 8.6/9.3; long rows against few channels run faster alone
+// there (8 x 4096 -> 1024 10.6/10.0 and 8.7/9.5, 8 x 8192 -> 2048 15.7/14.2 and 13.1/13.6).
 constexpr uint32_t kPairSmemBytes = (233472 - 2 * 1024) / 2;   // 228 KB per SM, 1 KB reserved per CTA
 constexpr uint32_t kSoloSmemBytes = 200 * 1024;
 constexpr uint32_t kPairShareBytes = 160 * 1024;               // largest weight share per CTA run in pairs

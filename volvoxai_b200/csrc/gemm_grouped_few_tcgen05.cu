@@ -11,8 +11,8 @@
 // 8 x 4096 -> 4096 9.7 (27.3), 64 x 4096 -> 14336 18.9 (28.2).
 //
 // A stage is 256 bytes of K: one TMA box of weights ([2 K blocks][channels x 128 B]), one of activations, one commit,
-// and the 1 .. 8 groups that lie in it, each in accumulator columns of its own, drained together.  The rings hold about
-// 200 KB per SM, which is what keeps the HBM stream going.
+// and the 1 .. 8 groups that lie in it, each in accumulator columns of its own, drained together.  The ring of a CTA holds
+// about 200 KB, which is what keeps the HBM stream going, half of that in the form below that leaves room for a second CTA.
 //
 //   warp 0        TMA producer, activations (waits for the launch before this one)
 //   warp 1        allocates TMEM; one lane issues the MMAs (of the short tiles every other stage's; another warp the rest)
@@ -37,9 +37,13 @@ constexpr uint32_t kMaxStages = 12, kMaxBufs = 4;
 // BM channels per tile, LT live token slots, MPG MMAs (32 bytes of K) per group
 template <uint32_t BM, uint32_t LT, uint32_t MPG> struct Few {
     static constexpr uint32_t NT = LT < 16 ? 16 : LT;               // token columns of the MMA
-    // Up to 16 tokens two CTAs fit an SM (half of its shared memory and TMEM each), so that the next launch's CTAs
-    // start their weights while this launch drains: 8 x 4096 -> 14336 17.3 -> 16.5 us.  The short tiles want the deep
-    // ring instead (8 x 4096 -> 4096 13.7 us, 14.6 with half of it).
+    // Up to 16 tokens of 128-channel tiles two CTAs fit an SM (half of its shared memory and TMEM each).  Between launches
+    // of prepared activations the next one's CTAs so start their weights while this launch drains.  Behind a row quantizer
+    // the GEMM before it has ended when this one starts, and half the ring is still the faster form; us from a graph / in a
+    // stream, this and the whole SM's ring per CTA: 8 x 4096 -> 14336 16.1/16.3 and 16.3/17.2, 16 x 4096 -> 14336 17.8/18.0
+    // and 18.6/18.9, 8 x 4096 -> 14336 at G = 32 19.5/19.9 and 20.7/21.2, 5 x 2048 -> 11008 9.1/9.8 and 9.2/9.9,
+    // 8 x 8192 -> 28672 51.4/52.2 and 51.4/52.0.  The short tiles want the deep ring (8 x 4096 -> 4096 13.7 us, 14.6 with
+    // half of it).
     static constexpr bool kTwo = BM == 128 && LT <= 16;
     static constexpr uint32_t kCtas = kTwo ? 2 : 1, kTmemCols = kTwo ? 256 : 512, kSmemBudget = (kTwo ? 110 : 216) * 1024;
     static constexpr uint32_t kDrainWarps = NT == 64 ? 8 : 4;

@@ -251,7 +251,9 @@ int vxb_plan(const VxbPlanQuery* query, VxbLaunchPlan* out, char* why, uint32_t 
                 // K (48 KB for 128 x 256 alone, 32 KB in a pair on 256 x 256, 24 KB on 256 x 128) or by the MMAs on
                 // them (512, 512, 256 clocks); a pair takes longer to set up.  In clocks, from K = 4096 -> 4096 with
                 // fp32 output: 512 rows 16.8 / 16.7 / 13.3 us, 1024 rows 17.1 / 17.8 / -, 2048 rows 29.3 / 27.4 / -
-                // (alone / pair / narrow pair).
+                // (alone / pair / narrow pair).  Held against all three at K 1664 .. 14336, 130 .. 4096 rows and N 1024 ..
+                // 11008, fp32 and int8 outputs: 254 of 274 calls get the fastest; the most that one loses is 6 % (int8,
+                // 777 x 1664 -> 11008: a pair 26.1 us, alone 24.6).
                 const uint32_t pair_rows = ceil_div(q.rows, 256);
                 const uint64_t kb = round_up(q.k, kKAlign) / kKAlign;
                 const uint64_t alone = 9300ull + 724ull * kb * ceil_div(tiles, sms);
