@@ -504,15 +504,15 @@ int check_common(const VxbContext* ctx, const VxbWeight* w, const void* x, const
 }
 
 // Whether the row quantizer lets the GEMM behind it in before its own wait (quantize.cu's wait_and_release): few
-// activations for a small weight, whose GEMM holds nothing up and is mostly set-up.  Replayed from a graph, us, early /
-// late: 6 x 640 -> 1472 5.9 / 6.6, 4 x 576 -> 1536 5.9 / 6.2, 8 x 576 -> 2050 6.0 / 6.6, 8 x 128 -> 576 5.1 / 6.3, 64 x 256 ->
-// 576 5.7 / 5.8, 16 x 1024 -> 1000 6.1 / 6.4; past the line 8 x 576 -> 3072 6.2 / 6.2, 33 x 576 -> 576 6.2 / 6.0, 64 x 1024 ->
-// 1000 7.0 / 6.5, and a layer of 8 rows and hidden 1024 29.0 / 28.4.  In a stream of calls both are paced by the host at
-// these sizes.  Longer rows against narrow weights (8 x 8192 -> 1024 14.1 / 15.9 from a graph, 15.6 / 14.1 in a stream;
-// 32 x 2048 -> 2048 8.2 / 9.3, 9.4 / 8.5) go with the stream, and with the layers measured there.
+// activations of short rows for a small weight, whose GEMM holds nothing up and is mostly set-up.  Replayed from a graph,
+// us, early / late: 6 x 640 -> 1472 5.9 / 6.6, 4 x 576 -> 1536 5.9 / 6.2, 8 x 576 -> 2050 6.0 / 6.6, 8 x 128 -> 576 5.1 / 6.3,
+// 64 x 256 -> 576 5.7 / 5.8; past the line 8 x 576 -> 3072 6.2 / 6.2, 33 x 576 -> 576 6.2 / 6.0, 64 x 1024 -> 1000 7.0 / 6.5.
+// In a stream of calls both are paced by the host at these sizes.  Longer rows go with the layers they are part of and with
+// streams, not with a graph that repeats one of them: 16 x 1024 -> 1000 6.1 / 6.4, but a layer of 8 rows and hidden 1024 29.0
+// / 28.4, and one of 7 rows, hidden 640 and attention 1024 30.0 / 29.2 in a stream; 8 x 8192 -> 1024 14.1 / 15.9 from a
+// graph, 15.6 / 14.1 in a stream; 32 x 2048 -> 2048 8.2 / 9.3 and 9.4 / 8.5.
 bool release_early(const VxbWeight* w, uint32_t rows) {
-    const uint64_t weight_bytes = (uint64_t)w->d_out * w->kpad;
-    return !w->group && (uint64_t)rows * w->kpad <= 16384u && weight_bytes < (w->kpad <= 768 ? 3u << 19 : 1u << 20);
+    return !w->group && w->kpad <= 768 && (uint64_t)rows * w->kpad <= 16384u && (uint64_t)w->d_out * w->kpad < (3u << 19);
 }
 
 int quantize_into_scratch(VxbContext* ctx, const VxbWeight* w, const float* x, uint32_t rows,
