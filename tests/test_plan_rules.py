@@ -57,11 +57,13 @@ def test_grouped_rows_up_to_64_have_the_weights_as_m(rows, n, tile):
     assert plan["id"] == "GROUPED_TCGEN05" and (plan["tile_rows"], plan["tile_columns"]) == tile
 
 
-@pytest.mark.parametrize("rows,k,per_row", [(64, 1024, 256), (128, 1024, 256), (148, 1024, 256), (149, 1024, 128), (296, 1024, 128), (297, 1024, 64), (592, 1024, 64),
-                                            (593, 1024, 32), (777, 576, 32), (300, 576, 64), (1184, 256, 32), (1185, 256, 8), (64, 124, 8), (64, 128, 32),
-                                            (148, 4096, 256), (149, 4096, 128), (8192, 4096, 128), (40, 8192, 256)])
+@pytest.mark.parametrize("rows,k,per_row", [(64, 1024, 256), (148, 1024, 256), (149, 1024, 128), (296, 1024, 128), (297, 1024, 64), (2368, 1024, 64),
+                                            (2369, 1024, 32), (777, 576, 32), (300, 576, 64), (592, 576, 64), (593, 576, 32), (4736, 256, 32), (4737, 256, 8),
+                                            (64, 124, 8), (64, 128, 32), (1184, 128, 32), (1185, 128, 8), (592, 4096, 256), (593, 4096, 128),
+                                            (40, 8192, 256)])
 def test_quantizer_threads_per_row(rows, k, per_row):
-    """Doubled while the launch stays within 256 threads per SM and a thread keeps a float4."""
+    """Doubled while the launch stays within 256 threads per SM and a thread keeps a float4, or within 1024 and it keeps four
+    (two at K up to 256)."""
     plan = pick(rows, k, 4096, fp32_input=True)
     assert plan["quantizer"] == 2 and plan["quantizer_grid"] == -(-rows // (256 // per_row))
 

@@ -555,16 +555,21 @@ uint32_t quantize_any_threads(uint32_t rows, uint32_t k) {
 }
 
 // ... with 128-bit loads: at most 8 float4 per thread, then doubled (from 8 to 32) while the whole launch stays within 256
-// threads per SM, 512 with the RMSNorm's longer row, and every thread keeps a float4.  More threads than that cost more in
-// row reductions and blocks than the loads in flight give, alone (us, never doubled / doubled from below 512 per SM to
-// below 1024 / this rule): 64 x 1024 2.1 / 1.8 / 1.8, 512 x 1024 2.2 / 2.8 / 2.1, 777 x 576 2.1 / 2.9 / 2.1, 2048 x 256
-// 2.2 / 2.8 / 2.1; with the norm 64 x 1024 4.9 / 2.7 / 2.7, 512 x 1024 5.2 / 4.2 / 3.3.
+// threads per SM and every thread keeps a float4, or within 1024 per SM and it keeps four (two at K up to 256); with the
+// RMSNorm's longer row within 512 per SM.  Chosen by the whole call (us, rows from memory, N = 2048): shorter shares cost row
+// reductions and blocks (300 x 1024 with 256 threads per row 10.4, with 64 10.2; 777 x 576 with 128 9.9, with 32 9.5; 1024 x
+// 256 with 64 8.7, with 32 8.1), fewer threads leave the GEMM's first loads beside rows still to come (2048 x 1024 with 64
+// 12.4, with 32 13.5; 4096 x 256 with 32 12.5, with 8 14.5; 1024 x 2048 with 128 13.8, with 64 14.7), although the quantizer
+// alone is then faster.  With the norm, alone: 64 x 1024 with 32 and 256 threads 4.9 and 2.7, 512 x 1024 with 256 4.2, with 128
+// 3.3.
 uint32_t quantize_vec_threads(uint32_t rows, uint32_t k, bool norm) {
-    const uint64_t most = 148u * (norm ? 512u : 256u);
+    const uint64_t few = 148u * (norm ? 512u : 256u), most = norm ? few : 148u * 1024u;
     uint32_t tpr = k <= 256 ? 8 : k <= 1024 ? 32 : k <= 2048 ? 64 : k <= 4096 ? 128 : 256;
     for (;;) {
         const uint32_t next = tpr == 8 ? 32u : 2u * tpr;
-        if (next > (uint32_t)kThreads || (uint64_t)rows * next > most || k / 4u < next) return tpr;
+        const uint64_t threads = (uint64_t)rows * next;
+        const uint32_t keep = threads <= few ? 1u : k <= 256 ? 2u : 4u;
+        if (next > (uint32_t)kThreads || threads > most || k / 4u < keep * next) return tpr;
         tpr = next;
     }
 }
